@@ -29,8 +29,8 @@ __device__ __forceinline__ double comp(R3 a, int d) { return d == 0 ? a.x : (d =
 // MahycoModule::produit
 __device__ __forceinline__ double produit(double A, double B, double C, double D) { return A * B - C * D; }
 // Arcane math::min / math::max
-__device__ __forceinline__ double amin(double a, double b) { return (a < b) ? a : b; }
-__device__ __forceinline__ double amax(double a, double b) { return (a < b) ? b : a; }
+__host__ __device__ __forceinline__ double amin(double a, double b) { return (a < b) ? a : b; }
+__host__ __device__ __forceinline__ double amax(double a, double b) { return (a < b) ? b : a; }
 // std::min / std::max
 __host__ __device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b : a; }
 __host__ __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b : a; }
@@ -228,6 +228,27 @@ __host__ __device__ __forceinline__ double div_rn(double x, double y) {
   if (x == 0.0 && y == y && y != 0.0) return std::signbit(x) != std::signbit(y) ? -0.0 : 0.0;
 #endif
   return x / y;
+}
+
+// Quotients of the pente-borne fluxes that are only read clamped: the
+// division is done where the clamped value depends on it.  With a finite,
+// nonzero divisor the comparisons of the operands tell exactly whether the
+// quotient is <= 0, or >= 1 (a real quotient >= 1 never rounds below 1).
+
+// amin(amax(0., a / b), 1.)
+__host__ __device__ __forceinline__ double pb_ratio01(double a, double b) {
+  const bool pos = b > 0., fin = fabs(b) <= 1.7976931348623157e308 && b != 0.;
+  if (fin && (pos ? a <= 0. : a >= 0.)) return 0.;
+  if (fin && (pos ? a >= b : a <= b)) return 1.;
+  return amin(amax(0., a / b), 1.);
+}
+
+// amin(amax(a / b - 1/2, -1/2), 1/2)
+__host__ __device__ __forceinline__ double pb_ratio_mid(double a, double b) {
+  const bool pos = b > 0., fin = fabs(b) <= 1.7976931348623157e308 && b != 0.;
+  if (fin && (pos ? a <= 0. : a >= 0.)) return -1. / 2.;
+  if (fin && (pos ? a >= b : a <= b)) return 1. / 2.;
+  return amin(amax(a / b - 1. / 2., -1. / 2.), 1. / 2.);
 }
 
 // limiter id as a template argument: 0-2 the classical limiters (one
