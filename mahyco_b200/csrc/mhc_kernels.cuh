@@ -1484,7 +1484,7 @@ __device__ __forceinline__ void body_lagrange_cells(const Mesh& M, const mhc_cas
   }
   double rho = m / V;
   double tau = 0.5 * (1.0 / rho_n + 1.0 / rho);
-  double divu = 1.0 / dt * (1.0 / rho - 1.0 / rho_n) / tau;
+  double divu = div_rn(1.0 / dt * (1.0 / rho - 1.0 / rho_n), tau);
   if (pure) {
     for (int q = 0; q < NE; ++q)
       if ((mask >> q) & 1) { rhoe[q] = rho; taue[q] = tau; }

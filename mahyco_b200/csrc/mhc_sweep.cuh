@@ -1382,11 +1382,14 @@ __device__ __forceinline__ void body_sweep_nodes_lanes(const Mesh& M, const Fiel
   // backward difference of a node is the forward difference of the node
   // before it (same operands), taken from the previous lane: an inner node
   // (id > 0) sits one lane after its back neighbour on the same line
+  const bool has_r = ok && lane < 31 && id < nn - 1;
   double g[3], g_l[3], g_r[3];
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
     g[q] = 0.;
-    const double gfw = LIM != LIM_ORDER1 ? div_rn(ph_r[q] - ph[q], x_r - x) : 0.;
+    // (not on lane 31 or at the end of a line: nothing reads those, and the
+    // lane's own value, 0 / 0, would take the division's slow path)
+    const double gfw = (LIM != LIM_ORDER1 && has_r) ? div_rn(ph_r[q] - ph[q], x_r - x) : 0.;
     const double gbw = __shfl_up_sync(FULL, gfw, 1);
     if (LIM != LIM_ORDER1 && inner) {
       if constexpr (LIM == LIM_GEN)
@@ -1662,11 +1665,13 @@ __device__ __forceinline__ void body_sweep_nodes_tile(const Mesh& M, const Field
       ph_r[q] = __shfl_down_sync(FULL, ph[q], 1);
     }
     const double bfm = __shfl_up_sync(FULL, ffm, 1);
+    // (nothing reads the difference of lane 31 or of the end of a line)
+    const bool has_r = ok && lane < 31 && id < nn - 1;
     double gr[3], g_l[3], g_r[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
       gr[q] = 0.;
-      const double gfw = LIM != LIM_ORDER1 ? div_rn(ph_r[q] - ph[q], x_r - x) : 0.;
+      const double gfw = (LIM != LIM_ORDER1 && has_r) ? div_rn(ph_r[q] - ph[q], x_r - x) : 0.;
       const double gbw = __shfl_up_sync(FULL, gfw, 1);
       if (LIM != LIM_ORDER1 && inner) gr[q] = limited_gradient_t<LIM>(gbw, gfw);
       g_l[q] = __shfl_up_sync(FULL, gr[q], 1);
