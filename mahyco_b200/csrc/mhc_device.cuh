@@ -104,6 +104,7 @@ struct Mesh {
   long long ncell, nnode;
   double o[3];         // origin
   double h[3];         // L/n per direction
+  int unit_normals;    // bit D: the initial outer normals along D are exactly -1 and 1 (mhc_sweep.cuh)
 };
 
 // linear ids in 32-bit arithmetic: a case has fewer than 2^31 nodes
@@ -137,7 +138,7 @@ __device__ __forceinline__ R3 node_x0(const Mesh& M, int i, int j, int k) {
 }
 
 // Hexa8 / Quad4 local node offsets
-__device__ __forceinline__ void local_node_offset(int l, int& di, int& dj, int& dk) {
+__host__ __device__ __forceinline__ void local_node_offset(int l, int& di, int& dj, int& dk) {
   di = (l == 1 || l == 2 || l == 5 || l == 6) ? 1 : 0;
   dj = (l == 2 || l == 3 || l == 6 || l == 7) ? 1 : 0;
   dk = (l >= 4) ? 1 : 0;
