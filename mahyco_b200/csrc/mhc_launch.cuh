@@ -194,16 +194,16 @@ __global__ void __launch_bounds__(CT) kb_init_nodes(const CaseDesc* __restrict__
 }
 
 // resident blocks per SM asked of the compiler for the Lagrange cell pass:
-// 3 (80 registers) spills a little but hides more of its loads than 2
+// 6 (80 registers) spills a little but hides more of its loads than 4
 // (124 registers, no spills)
 #ifndef MHC_LAG_MIN_BLOCKS
-#define MHC_LAG_MIN_BLOCKS 3
+#define MHC_LAG_MIN_BLOCKS 6
 #endif
 
 // resident blocks per SM asked of the compiler for the node pass (a latency
 // bound gather: more warps in flight hide more of it)
 #ifndef MHC_NODES_MIN_BLOCKS
-#define MHC_NODES_MIN_BLOCKS 4
+#define MHC_NODES_MIN_BLOCKS 8
 #endif
 
 // LAG: a Lagrangian run (no remap): last positions, pressure surfaces
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(CT, MHC_NODES_MIN_BLOCKS) kb_lagrange_nodes(co
 
 // resident blocks per SM asked of the compiler for the geometry pass
 #ifndef MHC_GEOM_MIN_BLOCKS
-#define MHC_GEOM_MIN_BLOCKS 1
+#define MHC_GEOM_MIN_BLOCKS 2
 #endif
 
 template <int DIM>
@@ -389,7 +389,7 @@ kb_sweep_nodes(const CaseDesc* __restrict__ C, PhaseList L, int k) {
 
 // remap finalize after K performed sweeps: cells read U[K&1], nodes Ud[(K-1)&1]
 #ifndef MHC_FIN_MIN_BLOCKS
-#define MHC_FIN_MIN_BLOCKS 3
+#define MHC_FIN_MIN_BLOCKS 6
 #endif
 
 template <int DIM, int NE, bool ADV = false>
