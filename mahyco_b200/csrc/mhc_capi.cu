@@ -84,7 +84,8 @@ int engine_rebuild(Engine* e) {
     e->desc_cap = std::max(nc, 2 * e->desc_cap);
     CK(cudaMallocAsync((void**)&e->d_desc, e->desc_cap * sizeof(CaseDesc), e->stream));
   }
-  std::vector<CaseDesc> desc(nc);
+  std::vector<CaseDesc>& desc = e->h_desc;
+  desc.resize(nc);
   for (int i = 0; i < nc; ++i) {
     mhc_case* h = e->cases[i];
     h->slot = i;
@@ -143,6 +144,7 @@ int engine_rebuild(Engine* e) {
         tot += (long long)gx * gy * gz;
       }
       L.total = (int)tot;
+      L.solo = L.n == 1 ? g.members[0] : -1;
       return tot <= INT_MAX;
     };
     bool ok = phase(g.init_cells, PH_CELLS) && phase(g.init_nodes, PH_NODES) && phase(g.lag_cells, PH_CELLS) &&
@@ -256,8 +258,8 @@ void launch_init(Engine* e) {
 
 template <int DIM, bool EL, bool HG, bool LAG, bool CSTS = false>
 void lag_nodes_launch(Engine* e, Group& g) {
-  plaunch(e, kb_lagrange_nodes<DIM, EL, HG, LAG, CSTS>, CT, 0, g.lag_nodes);
-  if (HG) plaunch(e, kb_hourglass<DIM>, CT, 0, g.lag_nodes);
+  plaunch_case(e, MHC_KERNEL(kb_lagrange_nodes<DIM, EL, HG, LAG, CSTS, SOLO>), CT, 0, g.lag_nodes);
+  if (HG) plaunch_case(e, MHC_KERNEL(kb_hourglass<DIM, SOLO>), CT, 0, g.lag_nodes);
 }
 
 // elasto-plasticity and the anti-hourglass correction come with Lagrangian
@@ -285,8 +287,8 @@ void launch_lagrange_nodes(Engine* e) {
     if (g.ADV) {
       // sans-lagrange: prescribed velocities (validated without cell
       // boundary conditions)
-      if (g.DIM == 2) plaunch(e, kb_advect_nodes<2>, CT, 0, g.lag_nodes);
-      else plaunch(e, kb_advect_nodes<3>, CT, 0, g.lag_nodes);
+      if (g.DIM == 2) plaunch_case(e, MHC_KERNEL(kb_advect_nodes<2, SOLO>), CT, 0, g.lag_nodes);
+      else plaunch_case(e, MHC_KERNEL(kb_advect_nodes<3, SOLO>), CT, 0, g.lag_nodes);
       continue;
     }
     if (g.DIM == 2) lag_nodes_dispatch<2>(e, g);
@@ -294,11 +296,11 @@ void launch_lagrange_nodes(Engine* e) {
     if (g.CBC) {
       // cell variables of the boundary conditions, after the node pass
       if (g.DIM == 2) {
-        plaunch(e, kb_node_bcs<2>, CT, 0, g.lag_nodes);
-        plaunch(e, kb_cell_bcs<2>, CT, 0, g.lag_cells);
+        plaunch_case(e, MHC_KERNEL(kb_node_bcs<2, SOLO>), CT, 0, g.lag_nodes);
+        plaunch_case(e, MHC_KERNEL(kb_cell_bcs<2, SOLO>), CT, 0, g.lag_cells);
       } else {
-        plaunch(e, kb_node_bcs<3>, CT, 0, g.lag_nodes);
-        plaunch(e, kb_cell_bcs<3>, CT, 0, g.lag_cells);
+        plaunch_case(e, MHC_KERNEL(kb_node_bcs<3, SOLO>), CT, 0, g.lag_nodes);
+        plaunch_case(e, MHC_KERNEL(kb_cell_bcs<3, SOLO>), CT, 0, g.lag_cells);
       }
     }
   }
@@ -310,24 +312,24 @@ void launch_lagrange_cells(Engine* e) {
     if (g.EL && g.EULER) {
       // elasto cases with the remap: the deviator and plastic strains packed
       // among the projected variables
-      if (g.DIM == 2) plaunch(e, kb_lagrange_cells<2, 1, true, true>, CT, 0, g.lag_cells);
-      else plaunch(e, kb_lagrange_cells<3, 1, true, true>, CT, 0, g.lag_cells);
+      if (g.DIM == 2) plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<2, 1, true, true, false, SOLO>), CT, 0, g.lag_cells);
+      else plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<3, 1, true, true, false, SOLO>), CT, 0, g.lag_cells);
     } else if (g.EL) {
       // elasto cases: one environment (validated at creation)
-      if (g.DIM == 2) plaunch(e, kb_lagrange_cells<2, 1, false, true>, CT, 0, g.lag_cells);
-      else plaunch(e, kb_lagrange_cells<3, 1, false, true>, CT, 0, g.lag_cells);
+      if (g.DIM == 2) plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<2, 1, false, true, false, SOLO>), CT, 0, g.lag_cells);
+      else plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<3, 1, false, true, false, SOLO>), CT, 0, g.lag_cells);
     } else if (g.CSTS) {
       // CSTS: the cell pass computes the geometry itself (it reads the
       // corner normals at n first), then the forward velocity update
-      DISPATCH_GROUP(g, (plaunch(e, kb_lagrange_cells<DIM_, NE_, true, false, true>, CT, 0, g.lag_cells)));
-      if (g.DIM == 2) plaunch(e, kb_csts_forward<2>, CT, 0, g.lag_nodes);
-      else plaunch(e, kb_csts_forward<3>, CT, 0, g.lag_nodes);
+      DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<DIM_, NE_, true, false, true, SOLO>), CT, 0, g.lag_cells)));
+      if (g.DIM == 2) plaunch_case(e, MHC_KERNEL(kb_csts_forward<2, SOLO>), CT, 0, g.lag_nodes);
+      else plaunch_case(e, MHC_KERNEL(kb_csts_forward<3, SOLO>), CT, 0, g.lag_nodes);
     } else {
-      if (g.DIM == 2) plaunch(e, kb_lagrange_geom<2>, CT, 0, g.lag_cells);
-      else plaunch(e, kb_lagrange_geom<3>, CT, 0, g.lag_cells);
-      if (g.ADV) DISPATCH_GROUP(g, (plaunch(e, kb_advect_cells<DIM_, NE_>, CT, 0, g.lag_cells)));
-      else if (g.EULER) DISPATCH_GROUP(g, (plaunch(e, kb_lagrange_cells<DIM_, NE_, true, false>, CT, 0, g.lag_cells)));
-      else DISPATCH_GROUP(g, (plaunch(e, kb_lagrange_cells<DIM_, NE_, false, false>, CT, 0, g.lag_cells)));
+      if (g.DIM == 2) plaunch_case(e, MHC_KERNEL(kb_lagrange_geom<2, SOLO>), CT, 0, g.lag_cells);
+      else plaunch_case(e, MHC_KERNEL(kb_lagrange_geom<3, SOLO>), CT, 0, g.lag_cells);
+      if (g.ADV) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_advect_cells<DIM_, NE_, SOLO>), CT, 0, g.lag_cells)));
+      else if (g.EULER) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<DIM_, NE_, true, false, false, SOLO>), CT, 0, g.lag_cells)));
+      else DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<DIM_, NE_, false, false, false, SOLO>), CT, 0, g.lag_cells)));
     }
   }
 }
@@ -373,17 +375,17 @@ void launch_remap_variables(Engine* e) {
     {
       StageTimer tm(e, MHC_STAGE_FINALIZE_CELLS);
       if (g.EULER == 2) {
-        if (g.DIM == 2) plaunch(e, kb_euler_volume<2>, CT, 0, g.fin_cells);
-        else plaunch(e, kb_euler_volume<3>, CT, 0, g.fin_cells);
+        if (g.DIM == 2) plaunch_case(e, MHC_KERNEL(kb_euler_volume<2, SOLO>), CT, 0, g.fin_cells);
+        else plaunch_case(e, MHC_KERNEL(kb_euler_volume<3, SOLO>), CT, 0, g.fin_cells);
       }
-      if (g.ADV) DISPATCH_GROUP(g, (plaunch(e, kb_remap_finalize_cells<DIM_, NE_, true>, CT, 0, g.fin_cells, K)));
-      else DISPATCH_GROUP(g, (plaunch(e, kb_remap_finalize_cells<DIM_, NE_>, CT, 0, g.fin_cells, K)));
+      if (g.ADV) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_remap_finalize_cells<DIM_, NE_, true, SOLO>), CT, 0, g.fin_cells, K)));
+      else DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_remap_finalize_cells<DIM_, NE_, false, SOLO>), CT, 0, g.fin_cells, K)));
     }
     {
       StageTimer tm(e, MHC_STAGE_FINALIZE_NODES);
-      if (K > 0 && g.ADV) DISPATCH_GROUP(g, (plaunch(e, kb_remap_finalize_nodes<DIM_, false>, CT, 0, g.fin_nodes, K)));
-      else if (K > 0) DISPATCH_GROUP(g, (plaunch(e, kb_remap_finalize_nodes<DIM_>, CT, 0, g.fin_nodes, K)));
-      if (g.EULER == 2) plaunch(e, kb_euler_axis_reset, CT, 0, g.fin_nodes);
+      if (K > 0 && g.ADV) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_remap_finalize_nodes<DIM_, false, SOLO>), CT, 0, g.fin_nodes, K)));
+      else if (K > 0) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_remap_finalize_nodes<DIM_, true, SOLO>), CT, 0, g.fin_nodes, K)));
+      if (g.EULER == 2) plaunch_case(e, MHC_KERNEL(kb_euler_axis_reset<SOLO>), CT, 0, g.fin_nodes);
     }
   }
 }
@@ -410,8 +412,8 @@ void launch_dt(Engine* e) {
     // whose remap ran reads the node speeds its node finalize pass stored
     int dirs[3];
     const bool spd = g.EULER == 1 && group_dirs(e, g, dirs) > 0 && spd_enabled();
-    if (!g.ADV && spd) DISPATCH_GROUP(g, (plaunch(e, kb_delta_t<DIM_, true>, CT, 0, g.dt)));
-    else if (!g.ADV) DISPATCH_GROUP(g, (plaunch(e, kb_delta_t<DIM_>, CT, 0, g.dt)));
+    if (!g.ADV && spd) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_delta_t<DIM_, true, SOLO>), CT, 0, g.dt)));
+    else if (!g.ADV) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_delta_t<DIM_, false, SOLO>), CT, 0, g.dt)));
     if (g.cases.n > 0) {
       kb_delta_t_finalize<<<cdiv(g.cases.n, 128), 128, 0, e->stream>>>(e->d_desc, e->d_ints + g.cases.off_cases, g.cases.n);
       ++e->launches;

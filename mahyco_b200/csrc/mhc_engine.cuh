@@ -8,6 +8,7 @@
 #include <cstdlib>
 #include <map>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/mahyco_b200.h"
@@ -65,6 +66,7 @@ struct DevList {
   size_t off_start = 0;
   int n = 0;             // member cases
   int total = 0;         // virtual blocks of all members
+  int solo = -1;         // engine slot of the only member (n = 1)
 };
 
 struct Group {
@@ -92,6 +94,7 @@ struct Engine {
   std::vector<mhc_case*> cases;
   CaseDesc* d_desc = nullptr;
   int desc_cap = 0;
+  std::vector<CaseDesc> h_desc;  // the same on the host: a launch over one case passes its descriptor by value
   int* d_ints = nullptr;   // case indices and block prefix sums of every list
   size_t ints_cap = 0;
   std::vector<Group> groups;
@@ -292,6 +295,25 @@ inline void plaunch(Engine* e, K kernel, int threads, size_t smem, const DevList
   ++e->launches;
 }
 
+
+// a phase kernel over a list: the instance that takes the descriptor by value
+// when the list holds one case, the one that reads the table otherwise.
+// `pick` (MHC_KERNEL) names both.
+#define MHC_KERNEL(...) [](auto solo_) { constexpr bool SOLO = decltype(solo_)::value; return __VA_ARGS__; }
+
+template <class Pick, class... Args>
+inline void plaunch_case(Engine* e, Pick pick, int threads, size_t smem, const DevList& L, Args... args) {
+  if (L.total <= 0) return;
+  const int sc = (e->cur_stage >= 0 && e->stage_scale[e->cur_stage] >= 0) ? e->stage_scale[e->cur_stage] : e->grid_scale;
+  const PhaseList pl{e->d_ints + L.off_cases, e->d_ints + L.off_start, L.n, L.total};
+  auto launch = [&](auto kernel, const auto& table) {
+    const int grid = sc == 0 ? L.total : std::min(L.total, resident_blocks(e, kernel, threads, smem) * sc);
+    kernel<<<grid, threads, smem, e->stream>>>(table, pl, args...);
+  };
+  if (L.solo >= 0) launch(pick(std::true_type{}), CaseTable<true>{e->h_desc[L.solo]});
+  else launch(pick(std::false_type{}), CaseTable<false>{e->d_desc});
+  ++e->launches;
+}
 
 #define DISPATCH_GROUP(g, CALL)                                   \
   do {                                                            \

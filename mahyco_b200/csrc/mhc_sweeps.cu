@@ -16,41 +16,44 @@ namespace {
 template <int DIM, int LIM>
 void cell_sweep_elasto(Engine* e, Group& g, int D, int k) {
   StageTimer tm(e, MHC_STAGE_SWEEP_CELLS);
-  if (D == 0) plaunch(e, kb_sweep_cells<DIM, 1, 0, LIM, MHC_ELASTO_XV>, SW_THREADS, 0, g.sw_cells[0], k);
-  else if (D == 1) plaunch(e, kb_sweep_cells<DIM, 1, 1, LIM, MHC_ELASTO_XV>, SW_THREADS, 0, g.sw_cells[1], k);
-  else if constexpr (DIM == 3) plaunch(e, kb_sweep_cells<DIM, 1, 2, LIM, MHC_ELASTO_XV>, SW_THREADS, 0, g.sw_cells[2], k);
+  if (D == 0) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, 1, 0, LIM, MHC_ELASTO_XV, SOLO>), SW_THREADS, 0, g.sw_cells[0], k);
+  else if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, 1, 1, LIM, MHC_ELASTO_XV, SOLO>), SW_THREADS, 0, g.sw_cells[1], k);
+  else if constexpr (DIM == 3) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, 1, 2, LIM, MHC_ELASTO_XV, SOLO>), SW_THREADS, 0, g.sw_cells[2], k);
 }
 
+// (no line chunks along x: every mask of such a layout is over D = 1, 2)
 template <int DIM, int NE, int LIM>
 void cell_sweep(Engine* e, Group& g, int D, int k) {
   StageTimer tm(e, MHC_STAGE_SWEEP_CELLS);
-  if (D == 0) plaunch(e, kb_sweep_cells<DIM, NE, 0, LIM>, SW_THREADS, 0, g.sw_cells[0], k);
-  else if (D == 1) plaunch(e, kb_sweep_cells<DIM, NE, 1, LIM>, SW_THREADS, 0, g.sw_cells[1], k);
-  else if constexpr (DIM == 3) plaunch(e, kb_sweep_cells<DIM, NE, 2, LIM>, SW_THREADS, 0, g.sw_cells[2], k);
+  if (D == 0) {
+    if constexpr (LIM < LIM_COLS) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 0, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[0], k);
+  } else if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 1, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[1], k);
+  else if constexpr (DIM == 3) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 2, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[2], k);
 }
 
 // y / z cell sweeps through the shared-memory tile
 template <int DIM, int NE, int LIM>
 void cell_sweep_tile(Engine* e, Group& g, int D, int k) {
   StageTimer tm(e, MHC_STAGE_SWEEP_CELLS);
-  if (D == 1) plaunch(e, kb_sweep_cells_tile<DIM, NE, 1, LIM>, SWT_THREADS, swt_smem_bytes(NE), g.sw_cells[1], k);
-  else if constexpr (DIM == 3) plaunch(e, kb_sweep_cells_tile<DIM, NE, 2, LIM>, SWT_THREADS, swt_smem_bytes(NE), g.sw_cells[2], k);
+  if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_cells_tile<DIM, NE, 1, LIM, SOLO>), SWT_THREADS, swt_smem_bytes(NE), g.sw_cells[1], k);
+  else if constexpr (DIM == 3) plaunch_case(e, MHC_KERNEL(kb_sweep_cells_tile<DIM, NE, 2, LIM, SOLO>), SWT_THREADS, swt_smem_bytes(NE), g.sw_cells[2], k);
 }
 
 // y / z node sweeps through the shared-memory tile
 template <int DIM, int NE, int LIM>
 void node_sweep_tile(Engine* e, Group& g, int D, int k) {
   StageTimer tm(e, MHC_STAGE_SWEEP_NODES);
-  if (D == 1) plaunch(e, kb_sweep_nodes_tile<DIM, NE, 1, LIM>, SWT_THREADS, SWTN_SMEM_BYTES, g.sw_nodes[1], k);
-  else if constexpr (DIM == 3) plaunch(e, kb_sweep_nodes_tile<DIM, NE, 2, LIM>, SWT_THREADS, SWTN_SMEM_BYTES, g.sw_nodes[2], k);
+  if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_nodes_tile<DIM, NE, 1, LIM, SOLO>), SWT_THREADS, SWTN_SMEM_BYTES, g.sw_nodes[1], k);
+  else if constexpr (DIM == 3) plaunch_case(e, MHC_KERNEL(kb_sweep_nodes_tile<DIM, NE, 2, LIM, SOLO>), SWT_THREADS, SWTN_SMEM_BYTES, g.sw_nodes[2], k);
 }
 
 template <int DIM, int NE, int LIM>
 void node_sweep(Engine* e, Group& g, int D, int k) {
   StageTimer tm(e, MHC_STAGE_SWEEP_NODES);
-  if (D == 0) plaunch(e, kb_sweep_nodes<DIM, NE, 0, LIM>, SW_THREADS, 0, g.sw_nodes[0], k);
-  else if (D == 1) plaunch(e, kb_sweep_nodes<DIM, NE, 1, LIM>, SW_THREADS, 0, g.sw_nodes[1], k);
-  else if constexpr (DIM == 3) plaunch(e, kb_sweep_nodes<DIM, NE, 2, LIM>, SW_THREADS, 0, g.sw_nodes[2], k);
+  if (D == 0) {
+    if constexpr (LIM < LIM_COLS) plaunch_case(e, MHC_KERNEL(kb_sweep_nodes<DIM, NE, 0, LIM, SOLO>), SW_THREADS, 0, g.sw_nodes[0], k);
+  } else if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_nodes<DIM, NE, 1, LIM, SOLO>), SW_THREADS, 0, g.sw_nodes[1], k);
+  else if constexpr (DIM == 3) plaunch_case(e, MHC_KERNEL(kb_sweep_nodes<DIM, NE, 2, LIM, SOLO>), SW_THREADS, 0, g.sw_nodes[2], k);
 }
 
 }  // namespace
