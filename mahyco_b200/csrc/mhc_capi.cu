@@ -306,30 +306,39 @@ void launch_lagrange_nodes(Engine* e) {
   }
 }
 
-void launch_lagrange_cells(Engine* e) {
+// the cell pass of a Lagrangian group; with_dt: of one case, the time step too
+template <int DIM, int NE, bool EL>
+void lag_cells_launch(Engine* e, Group& g, bool with_dt) {
+  if (with_dt) plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<DIM, NE, false, EL, false, SOLO, SOLO>), CT, 0, g.lag_cells);
+  else plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<DIM, NE, false, EL, false, false, SOLO>), CT, 0, g.lag_cells);
+}
+
+// with_dt: Lagrangian groups of one case compute their time step in the same
+// pass (whole iterations; launch_dt then leaves them out)
+void launch_lagrange_cells(Engine* e, bool with_dt) {
   StageTimer tm(e, MHC_STAGE_LAGRANGE_CELLS);
   for (Group& g : e->groups) {
     if (g.EL && g.EULER) {
       // elasto cases with the remap: the deviator and plastic strains packed
       // among the projected variables
-      if (g.DIM == 2) plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<2, 1, true, true, false, SOLO>), CT, 0, g.lag_cells);
-      else plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<3, 1, true, true, false, SOLO>), CT, 0, g.lag_cells);
+      if (g.DIM == 2) plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<2, 1, true, true, false, false, SOLO>), CT, 0, g.lag_cells);
+      else plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<3, 1, true, true, false, false, SOLO>), CT, 0, g.lag_cells);
     } else if (g.EL) {
       // elasto cases: one environment (validated at creation)
-      if (g.DIM == 2) plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<2, 1, false, true, false, SOLO>), CT, 0, g.lag_cells);
-      else plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<3, 1, false, true, false, SOLO>), CT, 0, g.lag_cells);
+      if (g.DIM == 2) lag_cells_launch<2, 1, true>(e, g, with_dt);
+      else lag_cells_launch<3, 1, true>(e, g, with_dt);
     } else if (g.CSTS) {
       // CSTS: the cell pass computes the geometry itself (it reads the
       // corner normals at n first), then the forward velocity update
-      DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<DIM_, NE_, true, false, true, SOLO>), CT, 0, g.lag_cells)));
+      DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<DIM_, NE_, true, false, true, false, SOLO>), CT, 0, g.lag_cells)));
       if (g.DIM == 2) plaunch_case(e, MHC_KERNEL(kb_csts_forward<2, SOLO>), CT, 0, g.lag_nodes);
       else plaunch_case(e, MHC_KERNEL(kb_csts_forward<3, SOLO>), CT, 0, g.lag_nodes);
     } else {
       if (g.DIM == 2) plaunch_case(e, MHC_KERNEL(kb_lagrange_geom<2, SOLO>), CT, 0, g.lag_cells);
       else plaunch_case(e, MHC_KERNEL(kb_lagrange_geom<3, SOLO>), CT, 0, g.lag_cells);
       if (g.ADV) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_advect_cells<DIM_, NE_, SOLO>), CT, 0, g.lag_cells)));
-      else if (g.EULER) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<DIM_, NE_, true, false, false, SOLO>), CT, 0, g.lag_cells)));
-      else DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<DIM_, NE_, false, false, false, SOLO>), CT, 0, g.lag_cells)));
+      else if (g.EULER) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_lagrange_cells<DIM_, NE_, true, false, false, false, SOLO>), CT, 0, g.lag_cells)));
+      else DISPATCH_GROUP(g, (lag_cells_launch<DIM_, NE_, false>(e, g, with_dt)));
     }
   }
 }
@@ -405,16 +414,17 @@ bool spd_enabled() {
   return v;
 }
 
-void launch_dt(Engine* e) {
+void launch_dt(Engine* e, bool lagrangian_done) {
   StageTimer tm(e, MHC_STAGE_DELTA_T);
   for (Group& g : e->groups) {
+    if (lagrangian_done && !g.EULER && g.dt.solo >= 0) continue;
     // sans-lagrange keeps deltat_init: no CFL reduction; a Full Euler group
     // whose remap ran reads the node speeds its node finalize pass stored
     int dirs[3];
     const bool spd = g.EULER == 1 && group_dirs(e, g, dirs) > 0 && spd_enabled();
-    if (!g.ADV && spd) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_delta_t<DIM_, true, SOLO>), CT, 0, g.dt)));
-    else if (!g.ADV) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_delta_t<DIM_, false, SOLO>), CT, 0, g.dt)));
-    if (g.cases.n > 0) {
+    if (!g.ADV && spd) DISPATCH_GROUP(g, (plaunch_case<true>(e, MHC_KERNEL(kb_delta_t<DIM_, true, SOLO>), CT, 0, g.dt)));
+    else if (!g.ADV) DISPATCH_GROUP(g, (plaunch_case<true>(e, MHC_KERNEL(kb_delta_t<DIM_, false, SOLO>), CT, 0, g.dt)));
+    if ((g.ADV || g.dt.solo < 0) && g.cases.n > 0) {
       kb_delta_t_finalize<<<cdiv(g.cases.n, 128), 128, 0, e->stream>>>(e->d_desc, e->d_ints + g.cases.off_cases, g.cases.n);
       ++e->launches;
     }
@@ -428,9 +438,10 @@ void end_cycle(Engine* e) {
 
 void launch_cycle(Engine* e) {
   launch_lagrange_nodes(e);
-  launch_lagrange_cells(e);
+  const bool with_dt = !e->timing;  // a timed cycle keeps the time step apart
+  launch_lagrange_cells(e, with_dt);
   launch_remap(e);
-  launch_dt(e);
+  launch_dt(e, with_dt);
   end_cycle(e);
 }
 
@@ -1206,7 +1217,7 @@ int mhc_update_elasticity_and_plasticity(mhc_case* h) { return expect(h, S_VISCO
 int mhc_update_energy_and_pressure(mhc_case* h) {
   int r = expect(h, S_ELASTO, S_ENERGY);
   if (r) return r;
-  launch_lagrange_cells(h->solo);
+  launch_lagrange_cells(h->solo, false);
   CK(cudaGetLastError());
   return MHC_OK;
 }
@@ -1221,7 +1232,7 @@ int mhc_remap_apply(mhc_case* h) { return mhc_remap(h); }
 int mhc_compute_delta_t(mhc_case* h) {
   int r = expect(h, S_REMAP, S_IDLE);
   if (r) return r;
-  launch_dt(h->solo);
+  launch_dt(h->solo, false);
   end_cycle(h->solo);
   CK(cudaGetLastError());
   return MHC_OK;

@@ -298,16 +298,18 @@ inline void plaunch(Engine* e, K kernel, int threads, size_t smem, const DevList
 
 // a phase kernel over a list: the instance that takes the descriptor by value
 // when the list holds one case, the one that reads the table otherwise.
-// `pick` (MHC_KERNEL) names both.
+// `pick` (MHC_KERNEL) names both.  STRIDED: the first one strides over the case
+// itself, a device full of blocks is enough.
 #define MHC_KERNEL(...) [](auto solo_) { constexpr bool SOLO = decltype(solo_)::value; return __VA_ARGS__; }
 
-template <class Pick, class... Args>
+template <bool STRIDED = false, class Pick, class... Args>
 inline void plaunch_case(Engine* e, Pick pick, int threads, size_t smem, const DevList& L, Args... args) {
   if (L.total <= 0) return;
   const int sc = (e->cur_stage >= 0 && e->stage_scale[e->cur_stage] >= 0) ? e->stage_scale[e->cur_stage] : e->grid_scale;
   const PhaseList pl{e->d_ints + L.off_cases, e->d_ints + L.off_start, L.n, L.total};
   auto launch = [&](auto kernel, const auto& table) {
-    const int grid = sc == 0 ? L.total : std::min(L.total, resident_blocks(e, kernel, threads, smem) * sc);
+    const int k = sc == 0 && STRIDED && L.solo >= 0 ? 1 : sc;
+    const int grid = k == 0 ? L.total : std::min(L.total, resident_blocks(e, kernel, threads, smem) * k);
     kernel<<<grid, threads, smem, e->stream>>>(table, pl, args...);
   };
   if (L.solo >= 0) launch(pick(std::true_type{}), CaseTable<true>{e->h_desc[L.solo]});

@@ -37,7 +37,7 @@ struct Scalars {
   unsigned long long dt_min_bits;  // running min of l/(c+vmax) as ordered bits
   long long iteration_limit;  // last iteration this case may run
   int status;        // ST_* flags
-  int pad;
+  unsigned dt_blocks;  // blocks of the CFL reduction that are done (bit 30: one met a NaN)
   unsigned int eref_first[4];  // Mie-Gruneisen, energie-ref 0: the first cell (reference order) of
                                // each environment with a nonzero initial energy
 };
@@ -1437,8 +1437,11 @@ __device__ __forceinline__ void advance_temperature(const mhc_env_params& o, dou
   T = (e - e_n) / o.specific_heat + Tn;
 }
 
+// A Lagrangian run's characteristic length and sound speed come back in
+// l_out and c_out for the time step (not set beyond the last cell).
 template <int DIM, int NE, bool EULER, bool EL = false, bool CSTS = false>
-__device__ __forceinline__ void body_lagrange_cells(const Mesh& M, const mhc_case_params& P, const Fields& F, int bx) {
+__device__ __forceinline__ void body_lagrange_cells(const Mesh& M, const mhc_case_params& P, const Fields& F, int bx,
+                                                    double& l_out, double& c_out) {
   constexpr bool GEO = EL || CSTS;
   long long c = bx * (long long)CT + threadIdx.x;
   if (c >= M.ncell) return;
@@ -1726,6 +1729,8 @@ __device__ __forceinline__ void body_lagrange_cells(const Mesh& M, const mhc_cas
       cg += (1. - option) * fe[q] * ce[q];
     }
   }
+  l_out = l;
+  c_out = cg;
   F.rho[c] = rho; F.e[c] = eg; F.p[c] = pg; F.c[c] = cg; F.q[c] = qg; F.V[c] = V; F.l[c] = l;
   if (NE > 1 && !pure) {
     for (int q = 0; q < NE; ++q) {
@@ -2287,43 +2292,123 @@ __device__ __forceinline__ void body_remap_finalize_nodes(const Mesh& M, const F
 // minimum, then one ordered-bits atomicMin per block.  The minimum of
 // non-NaN values does not depend on the reduction order.
 // ---------------------------------------------------------------------------
-template <int DIM, bool SPD = false>
-__device__ __forceinline__ void body_delta_t(const Mesh& M, const mhc_case_params& P, const Fields& F, int bx) {
-  long long c = bx * (long long)CT + threadIdx.x;
-  double dx = 1.7976931348623157e308;
-  if (c < M.ncell) {
+// the largest node speed of a cell (0 unless the remap is Full Euler)
+template <int DIM, bool SPD>
+__device__ __forceinline__ double cell_vmax(const Mesh& M, const mhc_case_params& P, const Fields& F, long long c) {
+  double vmax = 0.;
+  if (P.is_euler_scheme == MHC_EULER_FULL) {
     int i, j, k;
     cell_ijk(M, c, i, j, k);
-    double vmax = 0.;
-    if (P.is_euler_scheme == MHC_EULER_FULL) {
-      for (int l = 0; l < (DIM == 3 ? 8 : 4); ++l) {
-        int a, b, d;
-        local_node_offset(l, a, b, d);
-        long long n = node_id(M, i + a, j + b, k + d);
-        if (SPD) {
-          vmax = amax(__ldg(F.spd + n), vmax);  // stored by the node finalize pass of this iteration
-        } else {
-          double vx = F.vx[n], vy = F.vy[n], vz = F.vz[n];
-          vmax = amax(sqrt(vx * vx + vy * vy + vz * vz), vmax);
-        }
+    for (int q = 0; q < (DIM == 3 ? 8 : 4); ++q) {
+      int a, b, d;
+      local_node_offset(q, a, b, d);
+      const long long n = node_id(M, i + a, j + b, k + d);
+      if (SPD) {
+        vmax = amax(__ldg(F.spd + n), vmax);  // stored by the node finalize pass of this iteration
+      } else {
+        const double vx = F.vx[n], vy = F.vy[n], vz = F.vz[n];
+        vmax = amax(sqrt(vx * vx + vy * vy + vz * vz), vmax);
       }
     }
-    dx = F.l[c] / (F.c[c] + vmax);
-    if (!(dx >= 0.)) { atomicOr(&F.s->status, ST_NAN); dx = 1.7976931348623157e308; }
   }
+  return vmax;
+}
+
+// what the end of an iteration reads besides the minimum
+struct StepEnd {
+  double t, dt, cfl, deltat_max, deltat_min, final_time;
+  long long iteration;
+  unsigned long long min_seen;  // the minimum when the block started
+  __device__ __forceinline__ void load(const mhc_case_params& P, const Scalars* s) {
+    t = s->t; dt = s->dt; iteration = s->iteration;
+    min_seen = *(volatile const unsigned long long*)&s->dt_min_bits;
+    cfl = P.cfl; deltat_max = P.deltat_max; deltat_min = P.deltat_min; final_time = P.final_time;
+  }
+};
+
+// end of iteration: new deltat (the kept one without CFL reduction), stop
+// test, advance to the next iteration
+__device__ __forceinline__ void end_iteration(const StepEnd& E, Scalars* s, bool keep_dt, double dt_kept,
+                                              unsigned long long min_bits) {
+  double new_dt;
+  int status = 0;
+  if (keep_dt) {
+    new_dt = dt_kept;
+  } else {
+    new_dt = E.cfl * __longlong_as_double((long long)min_bits);
+    new_dt = amin(new_dt, 1.05 * E.dt);
+    new_dt = amin(new_dt, E.deltat_max);
+    if (new_dt < E.deltat_min) status |= ST_DT_UNDERFLOW;
+  }
+  const bool not_yet = E.t < E.final_time, finish = E.t > E.final_time, too_much = (E.t + new_dt) > E.final_time;
+  if ((not_yet && too_much) || finish) status |= ST_STOP;
+  if (status) s->status |= status;
+  s->t_done = E.t;
+  s->iteration_done = E.iteration;
+  s->dt_next = new_dt;
+  s->old_dt = E.dt;
+  s->dt = new_dt;
+  s->t = E.t + new_dt;
+  s->iteration = E.iteration + 1;
+  s->dt_min_bits = 0x7fefffffffffffffull;
+}
+
+// one block's share of the reduction (every thread of the block calls it; dx
+// of a thread without a cell is the largest double): its minimum goes into
+// dt_min_bits, and the last of the case's `blocks` blocks ends the iteration,
+// with the other scalars it needs loaded ahead (E).  A NaN is only flagged
+// once all blocks are done, and not over an error that the pass itself
+// raised; with a flag set the iteration does not end.
+__device__ __forceinline__ void delta_t_block(const mhc_case_params& P, const Fields& F, const StepEnd& E, double dx,
+                                              bool bad, unsigned blocks) {
   for (int o = 16; o > 0; o >>= 1) dx = fmin(dx, __shfl_xor_sync(0xffffffffu, dx, o));
-  __shared__ double red[32];
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) red[wid] = dx;
-  __syncthreads();
-  if (wid == 0) {
-    dx = (lane < CT / 32) ? red[lane] : 1.7976931348623157e308;
-    for (int o = 16; o > 0; o >>= 1) dx = fmin(dx, __shfl_xor_sync(0xffffffffu, dx, o));
-    // a block whose minimum is not below the one already there has nothing to
-    // add (a stale read only costs an atomic)
-    const unsigned long long bits = (unsigned long long)__double_as_longlong(dx);
-    if (lane == 0 && bits < *(volatile unsigned long long*)&F.s->dt_min_bits) atomicMin(&F.s->dt_min_bits, bits);
+  __shared__ double red[CT / 32];
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = dx;
+  const bool any_bad = __syncthreads_or(bad);
+  if (threadIdx.x != 0) return;
+#pragma unroll
+  for (int w = 1; w < CT / 32; ++w) dx = fmin(dx, red[w]);
+  Scalars* s = F.s;
+  constexpr unsigned BAD = 1u << 30;
+  // (a block whose minimum is not below the one already there adds nothing)
+  const unsigned long long own = (unsigned long long)__double_as_longlong(dx);
+  if (own < E.min_seen) atomicMin(&s->dt_min_bits, own);
+  if (any_bad) atomicOr(&s->dt_blocks, BAD);
+  __threadfence();
+  const unsigned done = atomicAdd(&s->dt_blocks, 1u);
+  if ((done & (BAD - 1)) != blocks - 1) return;
+  __threadfence();
+  const int status = *(volatile int*)&s->status;
+  const unsigned long long bits = *(volatile unsigned long long*)&s->dt_min_bits;
+  if (status == 0) {
+    if (done & BAD) s->status = ST_NAN;
+    else end_iteration(E, s, P.deltat_constant, P.deltat_init, bits);
   }
+  s->dt_blocks = 0;
+}
+
+// a block's share of a launch over several cases: only the minimum, and the
+// NaN flag; kb_delta_t_finalize ends the iterations (counting the blocks of
+// twenty cases' lists took 30 us where the two kernels take 17)
+__device__ __forceinline__ void delta_t_block_min(const Fields& F, double dx) {
+  if (!(dx >= 0.)) { atomicOr(&F.s->status, ST_NAN); dx = 1.7976931348623157e308; }
+  for (int o = 16; o > 0; o >>= 1) dx = fmin(dx, __shfl_xor_sync(0xffffffffu, dx, o));
+  __shared__ double red_min[CT / 32];
+  if ((threadIdx.x & 31) == 0) red_min[threadIdx.x >> 5] = dx;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+#pragma unroll
+  for (int w = 1; w < CT / 32; ++w) dx = fmin(dx, red_min[w]);
+  const unsigned long long own = (unsigned long long)__double_as_longlong(dx);
+  if (own < *(volatile unsigned long long*)&F.s->dt_min_bits) atomicMin(&F.s->dt_min_bits, own);
+}
+
+// the end of an iteration without CFL reduction (sans-lagrange), or after a
+// reduction over several cases
+__device__ __forceinline__ void body_delta_t_finalize(const mhc_case_params& P, const Fields& F) {
+  StepEnd E;
+  E.load(P, F.s);
+  end_iteration(E, F.s, P.sans_lagrange || P.deltat_constant, P.deltat_init, E.min_seen);
 }
 
 // standalone IEquationOfState::applyEOS(env) on the current state of the
@@ -2360,33 +2445,6 @@ __device__ __forceinline__ void body_eos_apply(const Mesh& M, const mhc_case_par
     cg += (1. - option) * f * F.ec[q * N + c];
   }
   F.p[c] = pg; F.c[c] = cg;
-}
-
-// end of iteration: new deltat, stop test, advance to the next iteration
-__device__ __forceinline__ void body_delta_t_finalize(const mhc_case_params& P, const Fields& F) {
-  Scalars* s = F.s;
-  double old = s->dt;
-  double new_dt;
-  if (P.sans_lagrange || P.deltat_constant) {
-    new_dt = P.deltat_init;
-  } else {
-    double minimum_aux = __longlong_as_double((long long)s->dt_min_bits);
-    new_dt = P.cfl * minimum_aux;
-    new_dt = amin(new_dt, 1.05 * old);
-    new_dt = amin(new_dt, P.deltat_max);
-    if (new_dt < P.deltat_min) s->status |= ST_DT_UNDERFLOW;
-  }
-  double stop = P.final_time;
-  bool not_yet = s->t < stop, finish = s->t > stop, too_much = (s->t + new_dt) > stop;
-  if ((not_yet && too_much) || finish) s->status |= ST_STOP;
-  s->t_done = s->t;
-  s->iteration_done = s->iteration;
-  s->dt_next = new_dt;
-  s->old_dt = old;
-  s->dt = new_dt;
-  s->t = s->t + new_dt;
-  s->iteration += 1;
-  s->dt_min_bits = 0x7fefffffffffffffull;
 }
 
 }  // namespace mhc

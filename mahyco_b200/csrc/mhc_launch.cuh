@@ -268,7 +268,12 @@ __global__ void __launch_bounds__(CT, MHC_GEOM_MIN_BLOCKS) kb_lagrange_geom(cons
   }
 }
 
-template <int DIM, int NE, bool EULER, bool EL, bool CSTS = false, bool SOLO = false>
+// DT (whole iterations of one Lagrangian case): computeDeltaT in the same pass,
+// from the length and sound speed still in registers and the velocities the
+// node pass left; the last block ends the iteration.  A pass of its own and
+// one more kernel for the scalars took 6.4 of the 21.0 us of an iteration on
+// 200 x 10 cells.  The entry points called one by one keep kb_delta_t.
+template <int DIM, int NE, bool EULER, bool EL, bool CSTS = false, bool DT = false, bool SOLO = false>
 __global__ void __launch_bounds__(CT, MHC_LAG_MIN_BLOCKS) kb_lagrange_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant__ PhaseList L) {
   MHC_FOR_ITEMS(L) {
     const WorkItem wi = item_at<PH_CELLS>(C, L, w_);
@@ -276,7 +281,24 @@ __global__ void __launch_bounds__(CT, MHC_LAG_MIN_BLOCKS) kb_lagrange_cells(cons
     if (!case_active(F)) continue;
     resolve_positions(F);
     const Mesh M = C.at(wi.c).M;
-    body_lagrange_cells<DIM, NE, EULER, EL, CSTS>(M, *C.at(wi.c).P, F, wi.x);
+    const mhc_case_params& P = *C.at(wi.c).P;
+    const long long c = wi.x * (long long)CT + threadIdx.x;
+    // everything the time step needs besides this pass's results, loaded ahead
+    StepEnd E;
+    double vmax = 0.;
+    if constexpr (DT) {
+      E.load(P, F.s);
+      if (c < M.ncell) vmax = cell_vmax<DIM, false>(M, P, F, c);
+    }
+    double l = 0., cs = 0.;
+    body_lagrange_cells<DIM, NE, EULER, EL, CSTS>(M, P, F, wi.x, l, cs);
+    if constexpr (DT) {
+      double dx = 1.7976931348623157e308;
+      if (c < M.ncell) dx = l / (cs + vmax);
+      const bool bad = !(dx >= 0.);
+      delta_t_block(P, F, E, bad ? 1.7976931348623157e308 : dx, bad, cdiv_i(M.ncell, CT));
+      __syncthreads();
+    }
   }
 }
 
@@ -529,21 +551,46 @@ __global__ void __launch_bounds__(CT) kb_euler_axis_reset(const __grid_constant_
   }
 }
 
-// SPD: the node speeds stored by the node finalize pass (remap cases)
+// SPD: the node speeds stored by the node finalize pass (remap cases).
+// One case: a block strides over the cells and joins the reduction once, so
+// the launch is a device full of blocks at most, and the last one ends the
+// iteration.  Several cases: one item at a time, each to its own case's
+// minimum; kb_delta_t_finalize follows.
 template <int DIM, bool SPD = false, bool SOLO = false>
 __global__ void __launch_bounds__(CT) kb_delta_t(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant__ PhaseList L) {
-  MHC_FOR_ITEMS(L) {
-    const WorkItem wi = item_at<PH_CELLS>(C, L, w_);
-    Fields F = C.at(wi.c).F;
-    if (!case_active(F)) continue;
-    resolve_positions(F);
-    const Mesh M = C.at(wi.c).M;
-    body_delta_t<DIM, SPD>(M, *C.at(wi.c).P, F, wi.x);
-    __syncthreads();
+  constexpr double TOP = 1.7976931348623157e308;
+  if constexpr (SOLO) {
+    const Fields& F = C.d.F;
+    if (!case_active(F)) return;
+    const Mesh& M = C.d.M;
+    const mhc_case_params& P = *C.d.P;
+    StepEnd E;
+    E.load(P, F.s);
+    double dx = TOP;
+    bool bad = false;
+    for (unsigned c = blockIdx.x * CT + threadIdx.x; c < (unsigned)M.ncell; c += gridDim.x * CT) {
+      const double d = F.l[c] / (F.c[c] + cell_vmax<DIM, SPD>(M, P, F, c));
+      if (d >= 0.) dx = fmin(dx, d);
+      else bad = true;
+    }
+    delta_t_block(P, F, E, dx, bad, gridDim.x);
+  } else {
+    MHC_FOR_ITEMS(L) {
+      const WorkItem wi = item_at<PH_CELLS>(C, L, w_);
+      const Fields F = C.at(wi.c).F;
+      if (!case_active(F)) continue;
+      const Mesh M = C.at(wi.c).M;
+      const long long c = wi.x * (long long)CT + threadIdx.x;
+      double dx = TOP;
+      if (c < M.ncell) dx = F.l[c] / (F.c[c] + cell_vmax<DIM, SPD>(M, *C.at(wi.c).P, F, c));
+      delta_t_block_min(F, dx);
+      __syncthreads();
+    }
   }
 }
 
-// one thread per case
+// the end of an iteration without CFL reduction (sans-lagrange), or after one
+// over several cases, one thread per case
 static __global__ void kb_delta_t_finalize(const CaseDesc* __restrict__ C, const int* __restrict__ cases, int n) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const CaseDesc& cd = C[cases[t]];
