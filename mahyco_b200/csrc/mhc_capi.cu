@@ -123,6 +123,7 @@ int engine_rebuild(Engine* e) {
       it = gidx.find(key);
     }
     e->groups[it->second].members.push_back(i);
+    if (h->P.conservation_energie_totale) e->groups[it->second].CET = 1;
   }
   // per group: member case indices, then for every phase the prefix sums
   // of the members' virtual blocks
@@ -381,21 +382,24 @@ void launch_remap_variables(Engine* e) {
     if (!g.EULER) continue;
     int dirs[3];
     int K = group_dirs(e, g, dirs);
-    {
-      StageTimer tm(e, MHC_STAGE_FINALIZE_CELLS);
-      if (g.EULER == 2) {
-        if (g.DIM == 2) plaunch_case(e, MHC_KERNEL(kb_euler_volume<2, SOLO>), CT, 0, g.fin_cells);
-        else plaunch_case(e, MHC_KERNEL(kb_euler_volume<3, SOLO>), CT, 0, g.fin_cells);
-      }
-      if (g.ADV) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_remap_finalize_cells<DIM_, NE_, true, SOLO>), CT, 0, g.fin_cells, K)));
-      else DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_remap_finalize_cells<DIM_, NE_, false, SOLO>), CT, 0, g.fin_cells, K)));
+    if (g.CET) side_join(e);
+    StageTimer tm(e, MHC_STAGE_FINALIZE_CELLS);
+    if (g.EULER == 2) {
+      if (g.DIM == 2) plaunch_case(e, MHC_KERNEL(kb_euler_volume<2, SOLO>), CT, 0, g.fin_cells);
+      else plaunch_case(e, MHC_KERNEL(kb_euler_volume<3, SOLO>), CT, 0, g.fin_cells);
     }
-    {
-      StageTimer tm(e, MHC_STAGE_FINALIZE_NODES);
-      if (K > 0 && g.ADV) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_remap_finalize_nodes<DIM_, false, SOLO>), CT, 0, g.fin_nodes, K)));
-      else if (K > 0) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_remap_finalize_nodes<DIM_, true, SOLO>), CT, 0, g.fin_nodes, K)));
-      if (g.EULER == 2) plaunch_case(e, MHC_KERNEL(kb_euler_axis_reset<SOLO>), CT, 0, g.fin_nodes);
-    }
+    if (g.ADV) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_remap_finalize_cells<DIM_, NE_, true, SOLO>), CT, 0, g.fin_cells, K)));
+    else DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_remap_finalize_cells<DIM_, NE_, false, SOLO>), CT, 0, g.fin_cells, K)));
+  }
+  side_join(e);
+  for (Group& g : e->groups) {
+    if (!g.EULER) continue;
+    int dirs[3];
+    int K = group_dirs(e, g, dirs);
+    StageTimer tm(e, MHC_STAGE_FINALIZE_NODES);
+    if (K > 0 && g.ADV) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_remap_finalize_nodes<DIM_, false, SOLO>), CT, 0, g.fin_nodes, K)));
+    else if (K > 0) DISPATCH_GROUP(g, (plaunch_case(e, MHC_KERNEL(kb_remap_finalize_nodes<DIM_, true, SOLO>), CT, 0, g.fin_nodes, K)));
+    if (g.EULER == 2) plaunch_case(e, MHC_KERNEL(kb_euler_axis_reset<SOLO>), CT, 0, g.fin_nodes);
   }
 }
 
@@ -453,12 +457,22 @@ int engine_cycle(Engine* e, int n) {
   return MHC_OK;
 }
 
-// CUDA graph of one rotation period: 6 iterations bring every 2D and 3D
-// group back to the same sweep order, so the same graph replays
+// iterations of the CUDA graph: one rotation period of the sweeps, which
+// brings every remapped group back to the same order (2 in 2D, 3 in 3D, 6 for
+// both).  The forked node sweeps make a graph's instantiation and destruction
+// dear (6 iterations in 2D: 0.46 and 0.31 ms), so it is no longer than it has
+// to be; a Lagrangian engine's, without forks, takes 6.
+int graph_period(const Engine* e) {
+  bool d2 = false, d3 = false;
+  for (const Group& g : e->groups)
+    if (g.EULER) (g.DIM == 2 ? d2 : d3) = true;
+  return d2 != d3 ? (d2 ? 2 : 3) : 6;
+}
+
 int engine_cycle_graph(Engine* e, int n) {
   int r = engine_rebuild(e);
   if (r) return r;
-  const int period = 6;
+  const int period = graph_period(e);
   while (n > 0 && e->cycles_since_build % period != 0) {
     launch_cycle(e);
     --n;
@@ -551,6 +565,13 @@ void engine_release(Engine* e) {
   if (e->d_gather) cudaFreeAsync(e->d_gather, e->stream);
   if (e->h_gather) { cudaStreamSynchronize(e->stream); pinned_put(e->h_gather, e->gather_cap * sizeof(Scalars)); }
   e->d_gather = nullptr; e->h_gather = nullptr; e->gather_cap = 0;
+  if (e->side) cudaStreamDestroy(e->side);  // joined by every remap: nothing of it is still awaited
+  if (e->fork_ev) cudaEventDestroy(e->fork_ev);
+  for (cudaEvent_t& ev : e->node_ev) {
+    if (ev) cudaEventDestroy(ev);
+    ev = nullptr;
+  }
+  e->side = nullptr; e->fork_ev = nullptr;
   if (e->stage_ev) { cudaEventSynchronize(e->stage_ev); cudaEventDestroy(e->stage_ev); }
   if (e->h_stage) pinned_put(e->h_stage, e->stage_cap);
   e->stage_ev = nullptr; e->h_stage = nullptr; e->stage_cap = 0;
@@ -594,6 +615,7 @@ long long count_doubles(const mhc_case_params* p, long long& ncell, long long& n
   const bool csts = p->schema_csts && p->with_projection;
   long long nodes = 4 + 6 + 10 + ((p->sans_lagrange || csts) ? 3 : 0) + (csts ? 3 : 0) + ((p->with_projection && p->is_euler_scheme == MHC_EULER_FULL && !p->sans_lagrange) ? 1 : 0);
   if (csts) cells += 1;
+  if (p->with_projection && !p->sans_lagrange) cells += ne;  // mass fluxes of every other sweep
   if (!p->with_projection && !p->sans_lagrange) cells += 2 * ne;  // temperature
   return cells * ncell + nodes * nnode;
 }
@@ -719,6 +741,7 @@ void case_free(mhc_case* h) {
     // stream-ordered frees: the work already queued that reads the case
     // runs first; only a private stream is waited for, before it goes
     for (void* p : h->allocs) cudaFreeAsync(p, h->stream);
+    for (void* p : h->scratch) cudaFreeAsync(p, h->stream);
     if (h->own_stream) {
       cudaStreamSynchronize(h->stream);
       cudaStreamDestroy(h->stream);
@@ -809,6 +832,13 @@ int case_alloc(const mhc_case_params* params, cudaStream_t stream, mhc_case** ou
     F.Ud[b] = (double*)alloc(5 * NN * sizeof(double));
   }
   F.mflux = (double*)alloc(h->NE * N * sizeof(double));
+  if (h->P.with_projection && !h->P.sans_lagrange) {
+    // the mass fluxes of every other sweep, while the node sweep reads the ones before
+    if (ok && cudaMallocAsync((void**)&F.mflux1, h->NE * N * sizeof(double), h->stream) == cudaSuccess) h->scratch.push_back(F.mflux1);
+    else ok = false;
+  } else {
+    F.mflux1 = F.mflux;
+  }
   if (h->P.env[0].elasto_model) {
     F.S = (double*)alloc(6 * N * sizeof(double));
     F.pl = (double*)alloc(3 * N * sizeof(double));
@@ -1147,7 +1177,10 @@ int case_time_history(mhc_case* h, cudaStream_t st, double* out) {
 
 int mhc::engine_rebuild_shared(Engine* e) { return engine_rebuild(e); }
 int mhc::solo_engine_shared(mhc_case* h) { return solo_engine(h); }
-void mhc::launch_remap_sweeps_shared(Engine* e) { launch_remap_sweeps(e); }
+void mhc::launch_remap_sweeps_shared(Engine* e) {
+  launch_remap_sweeps(e);
+  side_join(e);
+}
 void mhc::launch_remap_variables_shared(Engine* e) { launch_remap_variables(e); }
 int mhc::fetch_shared(cudaStream_t s, const void* dev, void* host, size_t bytes) { return fetch(s, dev, host, bytes); }
 

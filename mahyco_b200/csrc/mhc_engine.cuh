@@ -47,6 +47,7 @@ struct mhc_case {
   bool own_stream = false;
   std::vector<void*> allocs;
   std::vector<size_t> alloc_bytes;  // size of each allocation (checkpoints)
+  std::vector<void*> scratch;       // allocations that hold nothing between iterations (not checkpointed)
   // asynchronous status read-back: two pinned slots and their events
   Scalars* h_scal = nullptr;
   cudaEvent_t scal_ev[2] = {nullptr, nullptr};
@@ -81,6 +82,7 @@ struct Group {
   int NCOLS = 0;               // bit D: the same for the node sweep
   int ADV = 0;                 // sans-lagrange: prescribed velocities, no Lagrange phase, no dual projection
   int CSTS = 0;                // schema-csts with the remap: half-step velocity updates around the step
+  int CET = 0;                 // a member has conservation-energie-totale (finalize cells reads the dual variables)
   long long it0;               // iteration of the members when the lists were built
   std::vector<int> members;
   DevList init_cells, init_nodes, lag_nodes, lag_cells, fin_cells, fin_nodes, dt;
@@ -115,6 +117,12 @@ struct Engine {
   // per-phase override of grid_scale (-1 = use grid_scale), set by a tuner
   int stage_scale[MHC_NUM_STAGES] = {-1, -1, -1, -1, -1, -1, -1};
   int cur_stage = -1;  // phase being launched (StageTimer scope)
+  // side stream of the node sweeps (NodeFork), made at the first remap
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork_ev = nullptr;
+  cudaEvent_t node_ev[3] = {nullptr, nullptr, nullptr};  // after the node sweeps of sweep k
+  bool side_failed = false;
+  int forked = 0;  // sweeps of this remap whose node sweeps are on the side stream, not joined yet
   // layout of the y / z sweeps of classical-limiter cases, set by a caller
   // or the tuner (mhc_*_set_sweep_layout): 0 = by mesh size (the line-chunk
   // thresholds), 1 = warp per line, 2 = shared-memory tile, 3 = line chunks
@@ -153,6 +161,59 @@ struct StageTimer {
     e->stage_launches[stage] += 1;
   }
 };
+
+// The node sweep of a direction needs that direction's mass fluxes and the
+// node sweep before it; the next cell sweep, and the finalize pass of the
+// cells, need only the cell sweeps.  So the node sweeps run on a side stream
+// beside them: forked after their cell sweep, joined before the finalize pass
+// of the nodes (side_join).  The mass fluxes have two buffers, by the parity
+// of the sweep: the cell sweep k waits for the node sweep k - 2, which read
+// the buffer it writes (side_reuse).  Within the scope e->stream is the side
+// stream.  A timed cycle keeps one stream.
+struct NodeFork {
+  Engine* e;
+  cudaStream_t main;
+  int k;
+  bool on;
+  NodeFork(Engine* e_, int k_) : e(e_), main(e_->stream), k(k_), on(false) {
+    if (e->timing || e->side_failed) return;
+    if (!e->side) {
+      int prio = 0;
+      bool ok = cudaStreamGetPriority(main, &prio) == cudaSuccess &&
+                cudaStreamCreateWithPriority(&e->side, cudaStreamNonBlocking, prio) == cudaSuccess &&
+                cudaEventCreateWithFlags(&e->fork_ev, cudaEventDisableTiming) == cudaSuccess;
+      for (cudaEvent_t& ev : e->node_ev) ok = ok && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess;
+      if (!ok) {
+        cudaGetLastError();
+        e->side_failed = true;
+        return;
+      }
+    }
+    cudaEventRecord(e->fork_ev, main);
+    cudaStreamWaitEvent(e->side, e->fork_ev, 0);
+    e->stream = e->side;
+    on = true;
+  }
+  ~NodeFork() {
+    if (!on) return;
+    e->stream = main;
+    cudaEventRecord(e->node_ev[k], e->side);
+    e->forked = k + 1;
+  }
+};
+
+// before the cell sweep k: the node sweep that read its mass flux buffer
+inline void side_reuse(Engine* e, int k) {
+  if (k >= 2 && e->forked >= k - 1) cudaStreamWaitEvent(e->stream, e->node_ev[k - 2], 0);
+}
+
+// the main stream waits for every node sweep forked (the last one follows
+// the others on the side stream)
+inline void side_join(Engine* e) {
+  if (e->forked == 0) return;
+  cudaStreamWaitEvent(e->stream, e->node_ev[e->forked - 1], 0);
+  e->forked = 0;
+}
 
 // sweep instances of a case (the template argument LIM of kb_sweep_nodes /
 // kb_sweep_cells)

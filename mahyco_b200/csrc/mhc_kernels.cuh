@@ -8,7 +8,7 @@
 //                   v0 [3][nnode] (sans-lagrange: the prescribed velocities)
 //   Lagrangian pos  Xp[3] (previous cycle), Xn[3] (this cycle)
 //   remap           U[2][NV][ncell] (NV = 3*NE+1: volumes, masses, energies, pseudo*V)
-//                   mflux[NE][ncell] (cell mass flux of the current sweep)
+//                   mflux, mflux1 [NE][ncell] (cell mass flux of the even / odd sweeps)
 //                   Ud[2][5][nnode] (node momentum x3, mass, kinetic energy)
 // A cell holding exactly one environment keeps that environment's values in
 // the global slot (Arcane's pure-cell storage); env slots are read and
@@ -50,7 +50,8 @@ struct Fields {
   double* X[2][3];         // Lagrangian positions, alternating by iteration
   double *Xp[3], *Xn[3];   // X of the previous / current iteration (resolved per launch)
   double* U[2];
-  double* mflux;
+  double* mflux;           // cell mass fluxes of the sweep [nb_env][ncell]; mflux1: of the odd sweeps of a
+  double* mflux1;          // remap (the kernels of sweep k put theirs in mflux)
   double* Ud[2];
   double* S;               // elasto: stress deviator [6][ncell] (xx yy zz xy yz zx)
   double* cqs;             // corner normals of the last Lagrangian mesh [NBN][3][ncell]

@@ -339,6 +339,7 @@ kb_sweep_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant_
     Fields F = C.at(wi.c).F;
     if (!case_active(F)) continue;
     resolve_positions(F);
+    if (k & 1) F.mflux = F.mflux1;
     const mhc_case_params& P = *C.at(wi.c).P;
     SweepArgs A;
     A.Uin = (k & 1) ? F.U[1] : F.U[0];
@@ -372,6 +373,7 @@ kb_sweep_cells_tile(const __grid_constant__ CaseTable<SOLO> C, const __grid_cons
     Fields F = C.at(wi.c).F;
     if (!case_active(F)) continue;  // uniform over the block (one case per item)
     resolve_positions(F);
+    if (k & 1) F.mflux = F.mflux1;
     const mhc_case_params& P = *C.at(wi.c).P;
     SweepArgs A;
     A.Uin = (k & 1) ? F.U[1] : F.U[0];
@@ -399,6 +401,7 @@ kb_sweep_nodes_tile(const __grid_constant__ CaseTable<SOLO> C, const __grid_cons
     Fields F = C.at(wi.c).F;
     if (!case_active(F)) continue;  // uniform over the block (one case per item)
     resolve_positions(F);
+    if (k & 1) F.mflux = F.mflux1;
     const Mesh M = C.at(wi.c).M;
     const mhc_case_params& P = *C.at(wi.c).P;
     DualArgs A;
@@ -424,6 +427,7 @@ kb_sweep_nodes(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant_
     Fields F = C.at(wi.c).F;
     if (!case_active(F)) continue;
     resolve_positions(F);
+    if (k & 1) F.mflux = F.mflux1;
     const Mesh M = C.at(wi.c).M;
     const mhc_case_params& P = *C.at(wi.c).P;
     const int done = sweep_done_dirs<DIM>(M, P, F.s->iteration, k);

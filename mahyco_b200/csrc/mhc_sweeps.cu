@@ -62,6 +62,7 @@ void node_sweep(Engine* e, Group& g, int D, int k) {
 template <int DIM, int NE>
 void sweep_step_dn(Engine* e, Group& g, int D, int k) {
   const int cl = ((g.COLS >> D) & 1) ? LIM_COLS + g.CLIM : g.CLIM;
+  side_reuse(e, k);
   if (NE == 1 && g.EL && g.EULER) {
     if constexpr (NE == 1) {
       switch (g.CLIM) {
@@ -92,6 +93,7 @@ void sweep_step_dn(Engine* e, Group& g, int D, int k) {
     default: cell_sweep<DIM, NE, LIM_ORDER1>(e, g, D, k); break;
   }
   if (g.ADV) return;  // sans-lagrange: no dual projection (PrepareRemap.cc:211)
+  NodeFork fork(e, k);
   const int nl = ((g.NCOLS >> D) & 1) ? LIM_COLS + g.LIM : g.LIM;
   if (D > 0 && !((g.NCOLS >> D) & 1) && ((g.NTILE >> D) & 1)) {
     switch (g.LIM) {
