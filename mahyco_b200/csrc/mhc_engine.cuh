@@ -85,6 +85,14 @@ struct Group {
   int CET = 0;                 // a member has conservation-energie-totale (finalize cells reads the dual variables)
   long long it0;               // iteration of the members when the lists were built
   std::vector<int> members;
+  // the same launches as another group (their lists aside): kernels, members
+  // and the phase of the sweep rotation
+  bool same_launches(const Group& o) const {
+    return DIM == o.DIM && NE == o.NE && EULER == o.EULER && skip == o.skip && EL == o.EL && HG == o.HG &&
+           CBC == o.CBC && LIM == o.LIM && CLIM == o.CLIM && COLS == o.COLS && TILE == o.TILE && NTILE == o.NTILE &&
+           NCOLS == o.NCOLS && ADV == o.ADV && CSTS == o.CSTS && CET == o.CET && it0 % 6 == o.it0 % 6 &&
+           members == o.members;
+  }
   DevList init_cells, init_nodes, lag_nodes, lag_cells, fin_cells, fin_nodes, dt;
   DevList sw_cells[3], sw_nodes[3];
   DevList cases;               // offset into the case-index arena
@@ -100,7 +108,9 @@ struct Engine {
   int* d_ints = nullptr;   // case indices and block prefix sums of every list
   size_t ints_cap = 0;
   std::vector<Group> groups;
+  std::vector<int> h_ints;       // the int arena as last uploaded
   bool dirty = true;
+  bool graph_stale = false;      // a launch setting changed: the captured graph is not kept by a rebuild
   long long cycles_since_build = 0;
   int nsm = 0;
   // timing
