@@ -5,8 +5,9 @@
 // be compared with the CPU oracle operation by operation.  Vector operations
 // follow Arcane's Real3 helpers (component-wise, left-to-right sums).
 #pragma once
-#include <cstdint>
 #include <cmath>
+#include <cstdint>
+#include <cstring>
 
 namespace mhc {
 
@@ -317,46 +318,83 @@ __host__ __device__ __forceinline__ double limited_gradient_ref(double gb, doubl
   return g;
 }
 
-// The same value with one division for minmod and superbee.  With slopes of
-// opposite signs, or a zero one, both limiter values are +0 and each term
-// is a signed zero, so g = +0.  With same-sign slopes, let n be the slope of
-// larger magnitude and d the other: the ratio n / d is >= 1, and comparing
-// |n| with |d| and 2 |d| exactly (doubling is exact) tells which branch of
-// the limiter the correctly rounded ratios fall in (the bounds 1/2, 1 and 2
-// are representable, so rounding never crosses them): minmod gives 1 for
-// n / d and d / n itself for the other; superbee gives n / d (<= 2) and 1,
-// or 2 and 2 d / n (the ratio < 1/2).  Only the ratio the result depends on
-// is divided; the constant term is formed as the reference forms it
-// (0.5 (phi x)), so the sum is bit-identical.  Non-finite slopes take the
-// reference path.
+// The same value with one division for minmod and superbee, two for van Leer
+// instead of four.  With slopes of opposite signs, or a zero one, every
+// limiter value is +0 and each term is a signed zero, so g = +0.  With
+// same-sign slopes, let n be the slope of larger magnitude and d the other:
+// the ratio n / d is >= 1, and comparing |n| with |d| and 2 |d| exactly
+// (doubling is exact) tells which branch of the limiter the correctly rounded
+// ratios fall in (the bounds 1/2, 1 and 2 are representable, so rounding
+// never crosses them): minmod gives 1 for n / d and d / n itself for the
+// other; superbee gives n / d (<= 2) and 1, or 2 and 2 d / n (the ratio <
+// 1/2).  Only the ratio the result depends on is divided; the constant term
+// is formed as the reference forms it (0.5 (phi x)), so the sum is
+// bit-identical.  Non-finite slopes take the reference path.
 template <int LIM>
 __host__ __device__ __forceinline__ double limited_gradient_t(double gb, double gf) {
-  if (LIM != 0 && LIM != 1) return limited_gradient_ref<LIM>(gb, gf);
-  const double ab = fabs(gb), af = fabs(gf);
-  if (!(ab <= 1.7976931348623157e308 && af <= 1.7976931348623157e308)) return limited_gradient_ref<LIM>(gb, gf);
-  if (!((gb > 0. && gf > 0.) || (gb < 0. && gf < 0.))) return 0.;
-  const bool fbig = af >= ab;             // the forward slope is n
+  if (LIM > 2) return limited_gradient_ref<LIM>(gb, gf);
+  const bool fbig = fabs(gf) >= fabs(gb);  // the forward slope is n
   const double n = fbig ? gf : gb, d = fbig ? gb : gf;
-  double tn, td;                          // terms whose limiter argument is n / d, d / n
-  if (LIM == 0) {
-    // minmod: phi(n / d) = 1, phi(d / n) = d / n
-    tn = 0.5 * (1.0 * d);
-    td = 0.5 * (flux_limiter_t<LIM>(div_rn(d, n)) * n);
-  } else if (fabs(n) <= 2.0 * fabs(d)) {
-    // superbee, n / d in [1, 2]: phi(n / d) = n / d, phi(d / n) = 1
-    tn = 0.5 * (flux_limiter_t<LIM>(div_rn(n, d)) * d);
-    td = 0.5 * (1.0 * n);
-  } else {
-    // superbee, n / d > 2: phi(n / d) = 2, phi(d / n) = 2 d / n
-    tn = 0.5 * (2.0 * d);
-    td = 0.5 * (flux_limiter_t<LIM>(div_rn(d, n)) * n);
+  // both finite (a NaN fails one of the comparisons)
+  if (!(fabs(n) <= 1.7976931348623157e308 && fabs(d) <= fabs(n))) return limited_gradient_ref<LIM>(gb, gf);
+  if (!((n > 0. && d > 0.) || (n < 0. && d < 0.))) return 0.;
+  // the two terms are added in either order alike, the first onto 0 (which
+  // takes the sign of an underflowed one)
+  if (LIM == 2) {
+    // van Leer: both ratios are needed, and positive
+    const double rn = n / d, rd = d / n;
+    if (rd <= 0.) return limited_gradient_ref<LIM>(gb, gf);  // d / n underflowed
+    return 0. + 0.5 * ((2.0 * rn / (1.0 + rn)) * d) + 0.5 * ((2.0 * rd / (1.0 + rd)) * n);
   }
-  // the reference adds the term of gf / gb (divisor gb) first
-  double g = 0.;
-  if (fbig) { g += tn; g += td; }
-  else { g += td; g += tn; }
-  return g;
+  if (LIM == 0) {
+    // minmod: phi(n / d) = 1, phi(d / n) = d / n (within [0, 1])
+    return 0. + 0.5 * ((d / n) * n) + 0.5 * d;
+  }
+  // superbee, n / d in [1, 2]: phi(n / d) = n / d, phi(d / n) = 1; n / d > 2:
+  // phi(n / d) = 2, phi(d / n) = 2 d / n
+  const bool near = fabs(n) <= 2.0 * fabs(d);
+  const double num = near ? n : d, den = near ? d : n;
+  const double r = num / den, phi = near ? r : 2.0 * r, c = near ? n : 2.0 * d;
+  return 0. + 0.5 * (phi * den) + 0.5 * c;
 }
+
+// Several quotients by one divisor, each rounded as an IEEE division, from
+// one reciprocal (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): with y the
+// correctly rounded 1 / b, a corrected quotient q1 is within an ulp of a / b,
+// its remainder a - b q1 is exact in a fused multiply-add, and q1 + r y
+// rounds to the quotient.  That needs no overflow, underflow or subnormal on
+// the way: |b| within [2^-400, 2^400] (else y = 0 and nothing passes) and
+// |a| within [2^-500, 2^500], or a = 0 (the sign of a zero quotient may
+// differ).  Out of these ranges q() says so (ok) and the caller divides.  Five operations
+// on the FP64 units a quotient instead of about eleven with the zero test
+// (div_rn), and no slow path.
+struct SharedDivisor {
+  double b, y;
+  __host__ __device__ static __forceinline__ unsigned exponent(double x) {
+#ifdef __CUDA_ARCH__
+    return (unsigned)__double2hiint(x) & 0x7ff00000u;
+#else
+    uint64_t u;
+    memcpy(&u, &x, 8);
+    return (unsigned)(u >> 32) & 0x7ff00000u;
+#endif
+  }
+  __host__ __device__ __forceinline__ void set(double divisor) {
+    b = divisor;
+    const bool in = exponent(b) - ((1023u - 400u) << 20) <= (800u << 20);
+    y = in ? 1.0 / b : 0.0;
+  }
+  __host__ __device__ __forceinline__ double q(double a, bool& ok) const {
+    const double q0 = a * y;
+    const double q1 = fma(fma(-b, q0, a), y, q0);
+    const double q2 = fma(fma(-b, q1, a), y, q1);
+    const bool in = exponent(a) - ((1023u - 500u) << 20) <= (1000u << 20);
+    ok = ok && (in || a == 0.0) && y != 0.0;
+    return q2;
+  }
+};
+
 __device__ __forceinline__ double limited_gradient(int id, double gb, double gf) {
   double g = 0.;
   if (gb != 0.) g += 0.5 * (flux_limiter(id, gf / gb) * gb);

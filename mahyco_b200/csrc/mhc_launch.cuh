@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(CT) kb_hourglass(const __grid_constant__ CaseT
 // registers at 65536 / (SW_THREADS * value)); measured best on B200: 6 for
 // the cell sweeps (80 registers), 8 for the node sweeps (64 registers)
 #ifndef MHC_SW_MIN_BLOCKS_CELLS
-#define MHC_SW_MIN_BLOCKS_CELLS 6
+#define MHC_SW_MIN_BLOCKS_CELLS 8
 #endif
 #ifndef MHC_SW_MIN_BLOCKS_NODES
 #define MHC_SW_MIN_BLOCKS_NODES 8
@@ -362,7 +362,7 @@ kb_sweep_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant_
 // limiters, first order): SWT_THREADS threads, swt_smem_bytes(NE) of
 // dynamic shared memory
 #ifndef MHC_SWT_MIN_BLOCKS
-#define MHC_SWT_MIN_BLOCKS 3
+#define MHC_SWT_MIN_BLOCKS 4
 #endif
 template <int DIM, int NE, int D, int LIM, bool SOLO = false>
 __global__ void __launch_bounds__(SWT_THREADS, MHC_SWT_MIN_BLOCKS)
@@ -390,7 +390,7 @@ kb_sweep_cells_tile(const __grid_constant__ CaseTable<SOLO> C, const __grid_cons
 
 // node sweep along D = 1, 2 through a shared-memory tile
 #ifndef MHC_SWTN_MIN_BLOCKS
-#define MHC_SWTN_MIN_BLOCKS 3
+#define MHC_SWTN_MIN_BLOCKS 4
 #endif
 template <int DIM, int NE, int D, int LIM, bool SOLO = false>
 __global__ void __launch_bounds__(SWT_THREADS, MHC_SWTN_MIN_BLOCKS)
