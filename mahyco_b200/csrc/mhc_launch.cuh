@@ -410,6 +410,7 @@ kb_sweep_nodes_tile(const __grid_constant__ CaseTable<SOLO> C, const __grid_cons
     A.order = P.ordre_projection;
     A.limiter = P.projection_limiteur_id;
     A.simple_pente = P.projection_simple_pente;
+    A.energy = P.conservation_energie_totale;
     A.done_dirs = sweep_done_dirs<DIM>(M, P, F.s->iteration, k);
     body_sweep_nodes_tile<DIM, NE, D, LIM>(M, F, A, wi.x, wi.y, swtn_tile);
   }
@@ -437,6 +438,7 @@ kb_sweep_nodes(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant_
     A.order = P.ordre_projection;
     A.limiter = P.projection_limiteur_id;
     A.simple_pente = P.projection_simple_pente;
+    A.energy = P.conservation_energie_totale;
     A.done_dirs = done;
     if constexpr (LIM >= LIM_COLS) body_sweep_nodes_cols<DIM, NE, D, LIM - LIM_COLS>(M, F, A, wi.x, wi.y);
     else body_sweep_nodes_lanes<DIM, NE, D, LIM>(M, F, A, wi.x, wi.y);

@@ -392,6 +392,7 @@ __device__ __forceinline__ double lane_cell_width(const Mesh& M, const Fields& F
 template <int DIM, int D, int LIM>
 struct CellLane {
   bool ok, face_b, up_left;
+  bool odd;               // a factor is not finite, or a divisor out of range: nothing is left out
   SharedDivisor den, dx;  // the cell's divisor; distance to the centre of the cell behind
   double fu;              // (ordre-projection - 1) x distance from the upwind cell's centre to the back face
   double cB, cF;          // outer normal x normal velocity x length x deltat of the back / front face, 0 at the ends
@@ -415,6 +416,8 @@ struct CellLane {
     cF = face_f ? ondF * un_r * L_r * dt : 0.;
     den.set(divisor);
     dx.set(face_b ? dxb : 1.);
+    constexpr double TOP = 1.7976931348623157e308;
+    odd = den.y == 0. || dx.y == 0. || !(fabs(fu) <= TOP && fabs(cB) <= TOP && fabs(cF) <= TOP);
   }
 
   // fluxes of the variable of value u (0 on lanes without a cell) through the
@@ -422,14 +425,14 @@ struct CellLane {
   __device__ __forceinline__ bool fluxes(double u, double& fB, double& fF) const {
     constexpr unsigned FULL = 0xffffffffu;
     fB = fF = 0.;
-    if (!__any_sync(FULL, u != 0.)) return false;
+    if (!__any_sync(FULL, u != 0. || odd)) return false;
     bool fine = true;
     double phi = den.q(u, fine);
     if (__any_sync(FULL, !fine)) phi = div_rn(u, den.b);
     const double phi_l = __shfl_up_sync(FULL, phi, 1);
     const double diff = phi - phi_l;
     double up = up_left ? phi_l : phi;  // upwind value
-    if (LIM != LIM_ORDER1 && __any_sync(FULL, face_b && diff != 0.)) {
+    if (__any_sync(FULL, (LIM != LIM_ORDER1 && face_b && diff != 0.) || odd)) {
       fine = true;
       double gf = face_b ? dx.q(diff, fine) : 0.;
       if (__any_sync(FULL, !fine)) gf = face_b ? div_rn(diff, dx.b) : 0.;
@@ -441,7 +444,7 @@ struct CellLane {
         const double ym = first ? phi : phi_l, yp = last ? phi : phi_r;
         gr = ok ? generalized_gradient(limiter, gf_r, gf, yp, ym, hw, hw_r, hw_l, simple_pente) : 0.;
       } else {
-        gr = limited_gradient_t<LIM == LIM_ORDER1 ? 0 : LIM>(gf, gf_r);
+        gr = LIM != LIM_ORDER1 ? limited_gradient_t<LIM == LIM_ORDER1 ? 0 : LIM>(gf, gf_r) : 0.;
       }
       const double gr_l = __shfl_up_sync(FULL, gr, 1);
       up = up + fu * (up_left ? gr_l : gr);
@@ -1348,6 +1351,7 @@ struct DualArgs {
   int limiter;
   int simple_pente;    // projection-simple-pente (generalised limiters)
   int done_dirs;       // bit d: direction d already swept this cycle
+  int energy;          // conservation-energie-totale: the kinetic energy is projected too
 };
 
 __device__ __forceinline__ bool node_inner_dir(const Mesh& M, int i, int j, int k, int d) {
@@ -1356,157 +1360,200 @@ __device__ __forceinline__ bool node_inner_dir(const Mesh& M, int i, int j, int 
   return id > 0 && id < nn - 1;
 }
 
+// ---------------------------------------------------------------------------
+// One variable of a node sweep, one node per lane along D: its value, the
+// limited gradient and the two fluxes, the neighbours' by shuffles.  The
+// swept velocity component comes first (its values give the upwind lengths of
+// the others), then the other two, then, where the total energy is conserved,
+// the kinetic energy (no gradient); nothing else reads the kinetic energy, so
+// it is left out otherwise.  The quotients by the node mass and by
+// the distance of the nodes share a reciprocal each.
+// ---------------------------------------------------------------------------
+template <int D, int LIM>
+struct NodeLane {
+  bool ok, inner, was_inner, has_r;  // has_r: the next node is on the same line, in the warp
+  bool odd;                          // an upwind length is not finite, or the distance out of range
+  SharedDivisor mass, dx;            // projected mass before the sweep; distance to the next node
+  double x, x_l, x_r, ffm, bfm, dt;
+  double geo_f, geo_b;
+  int order2;
+  // generalised limiters
+  int limiter, simple_pente;
+  double h0, hm, hp;
+
+  // positions and mass fluxes of the neighbours (every lane of the warp)
+  __device__ __forceinline__ void set_line(double position, double front_flux, double m, int id, int nn) {
+    constexpr unsigned FULL = 0xffffffffu;
+    x = position;
+    ffm = front_flux;
+    x_l = __shfl_up_sync(FULL, x, 1);
+    x_r = __shfl_down_sync(FULL, x, 1);
+    // the mass flux through the back half-plane of a node is the front one
+    // of the node behind it
+    bfm = __shfl_up_sync(FULL, ffm, 1);
+    has_r = ok && (threadIdx.x % SW_LANES) < 31 && id < nn - 1;
+    mass.set(was_inner ? m : 1.);
+    dx.set(has_r ? x_r - x : 1.);
+    if constexpr (LIM == LIM_GEN) {
+      // dual cell widths (UtilesRemap.cc:51-63); a missing second neighbour
+      // gives a zero width
+      const double x_ll = __shfl_up_sync(FULL, x, 2), x_rr = __shfl_down_sync(FULL, x, 2);
+      const bool bb = id >= 2, ff = id + 2 < nn;
+      h0 = hm = hp = 0.;
+      h0 = 0.5 * (x_r - x_l);
+      if (!bb) {
+        if (ff) hp = 0.5 * (x_rr - x);
+      } else if (!ff) {
+        hm = 0.5 * (x - x_ll);
+      } else {
+        hm = 0.5 * (x - x_ll);
+        hp = 0.5 * (x_rr - x);
+      }
+    }
+  }
+  // the node's value of a variable: U / mass of a node that a sweep of this
+  // remap moved, the node's own value (v) otherwise
+  __device__ __forceinline__ double value(double U, double v) const {
+    constexpr unsigned FULL = 0xffffffffu;
+    bool fine = true;
+    double ph = was_inner ? mass.q(U, fine) : v;
+    if (__any_sync(FULL, !fine) && was_inner) ph = div_rn(U, mass.b);
+    return ph;
+  }
+  // the update of U for a variable of value ph: component t of the order D,
+  // then the others (t = 0 sets the upwind lengths), t = 3 the kinetic energy
+  __device__ __forceinline__ double update(int t, double ph, double U) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const double ph_l = __shfl_up_sync(FULL, ph, 1), ph_r = __shfl_down_sync(FULL, ph, 1);
+    if (t == 0) {
+      const double ufront = 0.5 * (ph + ph_r), uback = 0.5 * (ph_l + ph);
+      const int signfront = (ufront > 0) ? 1 : -1, signback = (uback > 0) ? 1 : -1;
+      geo_f = (signfront * (x_r - x) - dt * ufront);
+      geo_b = (signback * (x - x_l) - dt * uback);
+      constexpr double TOP = 1.7976931348623157e308;
+      odd = dx.y == 0. || !(fabs(geo_f) <= TOP && fabs(geo_b) <= TOP);
+    }
+    const bool fr = ffm < 0., bk = bfm > 0.;
+    double FV = fr ? ph_r : ph, BV = bk ? ph_l : ph;
+    const double diff = has_r ? ph_r - ph : 0.;
+    // a warp without differences has no gradients
+    if (__any_sync(FULL, (LIM != LIM_ORDER1 && t < 3 && diff != 0.) || odd)) {
+      // the backward difference of a node is the forward difference of the
+      // node before it (same operands)
+      bool fine = true;
+      double gfw = has_r ? dx.q(diff, fine) : 0.;
+      if (__any_sync(FULL, !fine)) gfw = has_r ? div_rn(diff, dx.b) : 0.;
+      const double gbw = __shfl_up_sync(FULL, gfw, 1);
+      double g = 0.;
+      if (LIM != LIM_ORDER1 && inner && t < 3) {  // limited gradients of inner nodes only
+        if constexpr (LIM == LIM_GEN) g = generalized_gradient(limiter, gfw, gbw, ph_r, ph_l, h0, hp, hm, simple_pente);
+        else g = limited_gradient_t<LIM == LIM_ORDER1 ? 0 : LIM>(gbw, gfw);
+      }
+      const double g_l = __shfl_up_sync(FULL, g, 1), g_r = __shfl_down_sync(FULL, g, 1);
+      FV = FV + order2 * (0.5 * (fr ? g_r : g) * geo_f);
+      BV = BV + order2 * (0.5 * (bk ? g_l : g) * geo_b);
+    }
+    double W = U + (bfm * BV - ffm * FV);
+    if (t < 3 && fabs(W) < 1.e-300) W = 0.;
+    return W;
+  }
+};
+
+// mass flux through the front half-plane of node (i, j, k): the faces of the
+// node plane in face id order, then the environments
+template <int DIM, int NE, int D>
+__device__ __forceinline__ double front_mass_flux(const Mesh& M, const Fields& F, int i, int j, int k, int id) {
+  const long long N = M.ncell;
+  const int ndc = D == 0 ? M.ncx : (D == 1 ? M.ncy : M.ncz);
+  double ffm = 0.;
+  if (id >= ndc) return ffm;
+  const double w = DIM == 2 ? .5 : .25;
+  // the cells behind and in front of the node along the transverse axes
+  constexpr bool T2 = DIM == 3;
+  const int t1 = D == 0 ? j : i, n1 = D == 0 ? M.ncy : M.ncx, t2 = D == 2 ? j : k, n2 = D == 2 ? M.ncy : M.ncz;
+  const unsigned s1 = D == 0 ? (unsigned)M.ncx : 1u, s2 = D == 2 ? (unsigned)M.ncx : (unsigned)M.ncx * (unsigned)M.ncy;
+  const bool lo1 = t1 > 0, hi1 = t1 < n1, lo2 = !T2 || t2 > 0, hi2 = T2 && t2 < n2;
+  // id of the cell in front along both (2D: along the first)
+  const unsigned cf = (unsigned)i + (unsigned)M.ncx * ((unsigned)j + (T2 ? (unsigned)M.ncy * (unsigned)k : 0u));
+  const unsigned c2 = T2 ? cf - s2 : cf;
+  auto add = [&](bool in, unsigned c) {
+    if (!in) return;
+#pragma unroll
+    for (int q = 0; q < NE; ++q) ffm += w * __ldg(F.mflux + q * N + c);
+  };
+  add(lo1 && lo2, c2 - s1);
+  add(hi1 && lo2, c2);
+  if (T2) {
+    add(lo1 && hi2, cf - s1);
+    add(hi1 && hi2, cf);
+  }
+  return ffm;
+}
+
+// a direction swept before moved node (i, j, k)
+template <int DIM>
+__device__ __forceinline__ bool node_was_inner(const Mesh& M, const DualArgs& A, int i, int j, int k) {
+  bool was = false;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d)
+    if (((A.done_dirs >> d) & 1) && node_inner_dir(M, i, j, k, d)) was = true;
+  return was;
+}
+
 template <int DIM, int NE, int D, int LIM>
 __device__ __forceinline__ void body_sweep_nodes_lanes(const Mesh& M, const Fields& F, const DualArgs& A,
                                                        int vbx, int vby) {
   constexpr unsigned FULL = 0xffffffffu;
-  const long long NN = M.nnode, N = M.ncell;
+  const long long NN = M.nnode;
   const int lane = threadIdx.x % SW_LANES, row = threadIdx.x / SW_LANES;
   const int nn = D == 0 ? M.nnx : (D == 1 ? M.nny : M.nnz);
   constexpr int HL = LIM == LIM_GEN ? 3 : 2;
   constexpr int NO = LIM == LIM_GEN ? NOUT_W : NOUT;
   if (sweep_warp_empty<D>(M.nnx, M.nny, M.nnz, NO, HL, vbx, vby, row)) return;  // whole warp leaves together
   int i, j, k, id, ta, tb;
-  const bool ok = sweep_lane<D>(M.nnx, M.nny, M.nnz, NO, HL, vbx, vby, lane, row, i, j, k, id, ta, tb);
-  const bool inner = ok && id > 0 && id < nn - 1;
-  const bool out = ok && lane >= HL && lane < HL + NO;
+  NodeLane<D, LIM> K;
+  K.ok = sweep_lane<D>(M.nnx, M.nny, M.nnz, NO, HL, vbx, vby, lane, row, i, j, k, id, ta, tb);
+  K.inner = K.ok && id > 0 && id < nn - 1;
+  const bool out = K.ok && lane >= HL && lane < HL + NO;
+  K.was_inner = false;
+  K.dt = F.s->dt;
+  K.order2 = LIM == LIM_ORDER1 ? 0 : A.order - 1;  // ordre-projection - 1
+  K.limiter = A.limiter;
+  K.simple_pente = A.simple_pente;
   long long n = 0;
-  double U[5] = {0., 0., 0., 0., 0.};
-  double ph[4] = {0., 0., 0., 0.};
-  double x = 0., ffm = 0.;
-  if (ok) {
+  double m = 1., x = 0., ffm = 0.;
+  if (K.ok) {
     n = node_id(M, i, j, k);
     x = __ldg(F.Xn[D] + n);
-    bool was_inner = false;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d)
-      if (((A.done_dirs >> d) & 1) && node_inner_dir(M, i, j, k, d)) was_inner = true;
-    if (A.Uin) {
-      if (was_inner || out) {
-#pragma unroll
-        for (int q = 0; q < 5; ++q) U[q] = __ldg(A.Uin + q * NN + n);
-      }
-    } else {
-      const double mn = __ldg(F.mn + n), vx = __ldg(F.vx + n), vy = __ldg(F.vy + n), vz = __ldg(F.vz + n);
-      U[0] = mn * vx; U[1] = mn * vy; U[2] = mn * vz; U[3] = mn;
-      U[4] = 0.5 * mn * (vx * vx + vy * vy + vz * vz);
+    K.was_inner = node_was_inner<DIM>(M, A, i, j, k);
+    m = A.Uin ? __ldg(A.Uin + 3 * NN + n) : __ldg(F.mn + n);
+    ffm = front_mass_flux<DIM, NE, D>(M, F, i, j, k, id);
+  }
+  K.set_line(x, ffm, m, id, nn);
+  double vel[3] = {0., 0., 0.}, mom[3] = {0., 0., 0.};
+  if (K.ok) {
+    if (!K.was_inner || !A.Uin || A.energy) {
+      vel[0] = __ldg(F.vx + n);
+      vel[1] = __ldg(F.vy + n);
+      vel[2] = __ldg(F.vz + n);
     }
-    if (was_inner) {
-      ph[0] = div_rn(U[0], U[3]); ph[1] = div_rn(U[1], U[3]); ph[2] = div_rn(U[2], U[3]);
-      ph[3] = div_rn(U[4], U[3]);
-    } else {
-      const double vx = __ldg(F.vx + n), vy = __ldg(F.vy + n), vz = __ldg(F.vz + n);
-      ph[0] = vx; ph[1] = vy; ph[2] = vz;
-      ph[3] = 0.5 * (vx * vx + vy * vy + vz * vz);
-    }
-    // mass flux through the front half-plane: faces of the node plane in
-    // face id order, then environments
-    const int ndc = D == 0 ? M.ncx : (D == 1 ? M.ncy : M.ncz);
-    if (id < ndc) {
-      const double w = DIM == 2 ? .5 : .25;
 #pragma unroll
-      for (int b2 = 0; b2 < (DIM == 3 ? 2 : 1); ++b2) {
-#pragma unroll
-        for (int b1 = 0; b1 < 2; ++b1) {
-          int ci = i, cj = j, ck = k;
-          const int t1 = b1 - 1, t2 = b2 - 1;
-          if (D == 0) { cj += t1; ck += (DIM == 3 ? t2 : 0); }
-          else if (D == 1) { ci += t1; ck += (DIM == 3 ? t2 : 0); }
-          else { ci += t1; cj += t2; }
-          if (ci < 0 || cj < 0 || ck < 0) continue;
-          if (D != 0 && ci >= M.ncx) continue;
-          if (D != 1 && cj >= M.ncy) continue;
-          if (DIM == 3 && D != 2 && ck >= M.ncz) continue;
-          const long long cf = cell_id(M, ci, cj, DIM == 3 ? ck : 0);
-#pragma unroll
-          for (int q = 0; q < NE; ++q) ffm += w * __ldg(F.mflux + q * N + cf);
-        }
-      }
-    }
-  }
-  // neighbours
-  const double x_l = __shfl_up_sync(FULL, x, 1), x_r = __shfl_down_sync(FULL, x, 1);
-  double ph_l[4], ph_r[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    ph_l[q] = __shfl_up_sync(FULL, ph[q], 1);
-    ph_r[q] = __shfl_down_sync(FULL, ph[q], 1);
-  }
-  const double bfm = __shfl_up_sync(FULL, ffm, 1);
-  // dual cell widths for the generalised limiters (UtilesRemap.cc:51-63);
-  // a missing second neighbour gives a zero width
-  double h0 = 0., hm = 0., hp = 0.;
-  if constexpr (LIM == LIM_GEN) {
-    const double x_ll = __shfl_up_sync(FULL, x, 2), x_rr = __shfl_down_sync(FULL, x, 2);
-    const bool bb = id >= 2, ff = id + 2 < nn;
-    h0 = 0.5 * (x_r - x_l);
-    if (!bb) {
-      if (ff) hp = 0.5 * (x_rr - x);
-    } else if (!ff) {
-      hm = 0.5 * (x - x_ll);
-    } else {
-      hm = 0.5 * (x - x_ll);
-      hp = 0.5 * (x_rr - x);
-    }
-  }
-  // limited gradients of the velocity components (inner nodes only).  The
-  // backward difference of a node is the forward difference of the node
-  // before it (same operands), taken from the previous lane: an inner node
-  // (id > 0) sits one lane after its back neighbour on the same line
-  const bool has_r = ok && lane < 31 && id < nn - 1;
-  double g[3], g_l[3], g_r[3];
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    g[q] = 0.;
-    // (not on lane 31 or at the end of a line: nothing reads those, and the
-    // lane's own value, 0 / 0, would take the division's slow path)
-    const double gfw = (LIM != LIM_ORDER1 && has_r) ? div_rn(ph_r[q] - ph[q], x_r - x) : 0.;
-    const double gbw = __shfl_up_sync(FULL, gfw, 1);
-    if (LIM != LIM_ORDER1 && inner) {
-      if constexpr (LIM == LIM_GEN)
-        g[q] = generalized_gradient(A.limiter, gfw, gbw, ph_r[q], ph_l[q], h0, hp, hm, A.simple_pente);
-      else
-        g[q] = limited_gradient_t<LIM>(gbw, gfw);
-    }
-    g_l[q] = __shfl_up_sync(FULL, g[q], 1);
-    g_r[q] = __shfl_down_sync(FULL, g[q], 1);
-  }
-  if (!out) return;
-  if (!inner) {
-#pragma unroll
-    for (int q = 0; q < 5; ++q) A.Uout[q * NN + n] = U[q];
-    return;
-  }
-  const double dt = F.s->dt;
-  const int order2 = LIM == LIM_ORDER1 ? 0 : A.order - 1;  // ordre-projection - 1
-  U[3] += bfm - ffm;
-  double FV[3], BV[3], FE, BE;
-  {
-    const double ufront = 0.5 * (ph[D] + ph_r[D]);
-    const int signfront = (ufront > 0) ? 1 : -1;
-    const bool fr = ffm < 0.;
-    const double geo = (signfront * (x_r - x) - dt * ufront);
-#pragma unroll
-    for (int q = 0; q < 3; ++q) FV[q] = (fr ? ph_r[q] : ph[q]) + order2 * (0.5 * (fr ? g_r[q] : g[q]) * geo);
-    FE = (fr ? ph_r[3] : ph[3]) + order2 * (0.5 * 0. * geo);
-  }
-  {
-    const double uback = 0.5 * (ph_l[D] + ph[D]);
-    const int signback = (uback > 0) ? 1 : -1;
-    const bool bk = bfm > 0.;
-    const double geo = (signback * (x - x_l) - dt * uback);
-#pragma unroll
-    for (int q = 0; q < 3; ++q) BV[q] = (bk ? ph_l[q] : ph[q]) + order2 * (0.5 * (bk ? g_l[q] : g[q]) * geo);
-    BE = (bk ? ph_l[3] : ph[3]) + order2 * (0.5 * 0. * geo);
+    for (int q = 0; q < 3; ++q) mom[q] = A.Uin ? __ldg(A.Uin + q * NN + n) : m * vel[q];
   }
 #pragma unroll
-  for (int q = 0; q < 3; ++q) U[q] += bfm * BV[q] - ffm * FV[q];
-  U[4] += bfm * BE - ffm * FE;
-#pragma unroll
-  for (int q = 0; q < 3; ++q)
-    if (fabs(U[q]) < 1.e-300) U[q] = 0.;
-#pragma unroll
-  for (int q = 0; q < 5; ++q) A.Uout[q * NN + n] = U[q];
+  for (int t = 0; t < 3; ++t) {
+    constexpr int order[3] = {D, D == 0 ? 1 : 0, D == 2 ? 1 : 2};  // swept component first
+    const int q = order[t];
+    const double W = K.update(t, K.value(mom[q], vel[q]), mom[q]);
+    if (out) A.Uout[q * NN + n] = K.inner ? W : mom[q];
+  }
+  if (A.energy) {
+    const double vv = vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2];
+    const double U = !K.ok ? 0. : (A.Uin ? __ldg(A.Uin + 4 * NN + n) : 0.5 * m * vv);
+    const double W = K.update(3, K.value(U, 0.5 * vv), U);
+    if (out) A.Uout[4 * NN + n] = K.inner ? W : U;
+  }
+  if (out) A.Uout[3 * NN + n] = K.inner ? m + (K.bfm - K.ffm) : m;
 }
 
 // ---------------------------------------------------------------------------
@@ -1677,19 +1724,21 @@ __device__ __forceinline__ void body_sweep_nodes_cols(const Mesh& M, const Field
 // layout writes the updated variables of the written nodes (NOUT per
 // window).
 // ---------------------------------------------------------------------------
-constexpr int SWTN_SLOTS = 11;  // x, U[5], phi[4], front mass flux
+// staged: x, front mass flux, mass, then U and value of every variable
+// (1: a direction swept before moved the node, so its mass divides)
+constexpr int SWTN_SLOTS = 11;
 constexpr int SWTN_SMEM_BYTES = SWTN_SLOTS * SWT_FIELD * 8;
 
 template <int DIM, int NE, int D, int LIM>
 __device__ __forceinline__ void body_sweep_nodes_tile(const Mesh& M, const Fields& F, const DualArgs& A, int vbx,
                                                       int vby, double* __restrict__ sm) {
   static_assert(D >= 1, "x sweeps use the lane layout");
-  constexpr unsigned FULL = 0xffffffffu;
-  constexpr int S_X = 0, S_U = 1, S_PH = 6, S_FFM = 10;
+  constexpr int S_X = 0, S_FFM = 1, S_M = 2, S_U = 3, S_V = 7;
   const long long NN = M.nnode;
   const int nn = D == 1 ? M.nny : M.nnz, nb = D == 1 ? M.nnz : M.nny;
   const int x0 = vbx * SWT_COLS;
   const int g0 = vby * NOUT - 2;  // first position of the window (2 halo nodes)
+  const int nc = A.energy ? 4 : 3;
   // -- 1. load (row layout)
   {
     const int col = threadIdx.x % SWT_COLS, pos = threadIdx.x / SWT_COLS;
@@ -1697,16 +1746,23 @@ __device__ __forceinline__ void body_sweep_nodes_tile(const Mesh& M, const Field
     if (i < M.nnx && g >= 0 && g < nb * nn) {
       const int tb = (int)((unsigned)g / (unsigned)nn), id = g - tb * nn;
       const int j = D == 1 ? id : tb, k = D == 1 ? tb : id;
-      double ph[4], x, ffm, U[5];
-      node_state<DIM, NE, D>(M, F, A, i, j, k, id, ph, x, ffm);
-      node_u(F, A, NN, node_id(M, i, j, k), U);
+      const long long n = node_id(M, i, j, k);
       double* s = sm + pos * SWT_PITCH + col;
-      s[S_X * SWT_FIELD] = x;
+      const double m = A.Uin ? __ldg(A.Uin + 3 * NN + n) : __ldg(F.mn + n);
+      const double v[3] = {__ldg(F.vx + n), __ldg(F.vy + n), __ldg(F.vz + n)};
+      s[S_X * SWT_FIELD] = __ldg(F.Xn[D] + n);
+      s[S_FFM * SWT_FIELD] = front_mass_flux<DIM, NE, D>(M, F, i, j, k, id);
+      s[S_M * SWT_FIELD] = m;
 #pragma unroll
-      for (int q = 0; q < 5; ++q) s[(S_U + q) * SWT_FIELD] = U[q];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) s[(S_PH + q) * SWT_FIELD] = ph[q];
-      s[S_FFM * SWT_FIELD] = ffm;
+      for (int q = 0; q < 3; ++q) {
+        s[(S_V + q) * SWT_FIELD] = v[q];
+        s[(S_U + q) * SWT_FIELD] = A.Uin ? __ldg(A.Uin + q * NN + n) : m * v[q];
+      }
+      if (nc == 4) {
+        const double vv = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+        s[(S_V + 3) * SWT_FIELD] = 0.5 * vv;
+        s[(S_U + 3) * SWT_FIELD] = A.Uin ? __ldg(A.Uin + 4 * NN + n) : 0.5 * m * vv;
+      }
     }
   }
   __syncthreads();
@@ -1714,73 +1770,32 @@ __device__ __forceinline__ void body_sweep_nodes_tile(const Mesh& M, const Field
   const int lane = threadIdx.x % SW_LANES, w = threadIdx.x / SW_LANES;
   if (x0 + w < M.nnx && g0 < nb * nn) {  // warp-uniform
     const int g = g0 + lane;
-    const bool ok = g >= 0 && g < nb * nn;
-    const int id = ok ? g - (int)((unsigned)g / (unsigned)nn) * nn : 0;
-    const bool inner = ok && id > 0 && id < nn - 1;
-    const bool out = ok && lane >= 2 && lane < 2 + NOUT;
+    NodeLane<D, LIM> K;
+    K.ok = g >= 0 && g < nb * nn;
+    const int tb = K.ok ? (int)((unsigned)g / (unsigned)nn) : 0, id = K.ok ? g - tb * nn : 0;
+    K.inner = K.ok && id > 0 && id < nn - 1;
+    K.was_inner = K.ok && node_was_inner<DIM>(M, A, x0 + w, D == 1 ? id : tb, D == 1 ? tb : id);
+    K.dt = F.s->dt;
+    K.order2 = LIM == LIM_ORDER1 ? 0 : A.order - 1;  // ordre-projection - 1
+    const bool out = K.ok && lane >= 2 && lane < 2 + NOUT;
     double* s = sm + lane * SWT_PITCH + w;
-    double U[5] = {0., 0., 0., 0., 0.}, ph[4] = {0., 0., 0., 0.}, x = 0., ffm = 0.;
-    if (ok) {
+    double m = 1., x = 0., ffm = 0.;
+    if (K.ok) {
+      m = s[S_M * SWT_FIELD];
       x = s[S_X * SWT_FIELD];
-#pragma unroll
-      for (int q = 0; q < 5; ++q) U[q] = s[(S_U + q) * SWT_FIELD];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) ph[q] = s[(S_PH + q) * SWT_FIELD];
       ffm = s[S_FFM * SWT_FIELD];
     }
-    const double x_l = __shfl_up_sync(FULL, x, 1), x_r = __shfl_down_sync(FULL, x, 1);
-    double ph_l[4], ph_r[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      ph_l[q] = __shfl_up_sync(FULL, ph[q], 1);
-      ph_r[q] = __shfl_down_sync(FULL, ph[q], 1);
-    }
-    const double bfm = __shfl_up_sync(FULL, ffm, 1);
-    // (nothing reads the difference of lane 31 or of the end of a line)
-    const bool has_r = ok && lane < 31 && id < nn - 1;
-    double gr[3], g_l[3], g_r[3];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      gr[q] = 0.;
-      const double gfw = (LIM != LIM_ORDER1 && has_r) ? div_rn(ph_r[q] - ph[q], x_r - x) : 0.;
-      const double gbw = __shfl_up_sync(FULL, gfw, 1);
-      if (LIM != LIM_ORDER1 && inner) gr[q] = limited_gradient_t<LIM>(gbw, gfw);
-      g_l[q] = __shfl_up_sync(FULL, gr[q], 1);
-      g_r[q] = __shfl_down_sync(FULL, gr[q], 1);
-    }
-    if (out && inner) {
-      const double dt = F.s->dt;
-      const int order2 = LIM == LIM_ORDER1 ? 0 : A.order - 1;  // ordre-projection - 1
-      U[3] += bfm - ffm;
-      double FV[3], BV[3], FE, BE;
-      {
-        const double ufront = 0.5 * (ph[D] + ph_r[D]);
-        const int signfront = (ufront > 0) ? 1 : -1;
-        const bool fr = ffm < 0.;
-        const double geo = (signfront * (x_r - x) - dt * ufront);
-#pragma unroll
-        for (int q = 0; q < 3; ++q) FV[q] = (fr ? ph_r[q] : ph[q]) + order2 * (0.5 * (fr ? g_r[q] : gr[q]) * geo);
-        FE = (fr ? ph_r[3] : ph[3]) + order2 * (0.5 * 0. * geo);
-      }
-      {
-        const double uback = 0.5 * (ph_l[D] + ph[D]);
-        const int signback = (uback > 0) ? 1 : -1;
-        const bool bk = bfm > 0.;
-        const double geo = (signback * (x - x_l) - dt * uback);
-#pragma unroll
-        for (int q = 0; q < 3; ++q) BV[q] = (bk ? ph_l[q] : ph[q]) + order2 * (0.5 * (bk ? g_l[q] : gr[q]) * geo);
-        BE = (bk ? ph_l[3] : ph[3]) + order2 * (0.5 * 0. * geo);
-      }
-#pragma unroll
-      for (int q = 0; q < 3; ++q) U[q] += bfm * BV[q] - ffm * FV[q];
-      U[4] += bfm * BE - ffm * FE;
-#pragma unroll
-      for (int q = 0; q < 3; ++q)
-        if (fabs(U[q]) < 1.e-300) U[q] = 0.;
-#pragma unroll
-      for (int q = 0; q < 5; ++q) s[(S_U + q) * SWT_FIELD] = U[q];  // the lane's own slots
-    }
-    // outer nodes (not inner) keep their staged U
+    K.set_line(x, ffm, m, id, nn);
+    auto component = [&](int t, int q) {
+      const double U = K.ok ? s[(S_U + q) * SWT_FIELD] : 0., v = K.ok ? s[(S_V + q) * SWT_FIELD] : 0.;
+      const double W = K.update(t, K.value(U, v), U);
+      if (out && K.inner) s[(S_U + q) * SWT_FIELD] = W;  // the lane's own slots; outer nodes keep their U
+    };
+    component(0, D);  // swept component first
+    component(1, 0);
+    component(2, D == 2 ? 1 : 2);
+    if (nc == 4) component(3, 3);
+    if (out && K.inner) s[S_M * SWT_FIELD] = m + (K.bfm - K.ffm);
   }
   __syncthreads();
   // -- 3. store (row layout), written positions only
@@ -1792,7 +1807,9 @@ __device__ __forceinline__ void body_sweep_nodes_tile(const Mesh& M, const Field
       const long long n = node_id(M, i, D == 1 ? id : tb, D == 1 ? tb : id);
       const double* s = sm + pos * SWT_PITCH + col;
 #pragma unroll
-      for (int q = 0; q < 5; ++q) A.Uout[q * NN + n] = s[(S_U + q) * SWT_FIELD];
+      for (int q = 0; q < 3; ++q) A.Uout[q * NN + n] = s[(S_U + q) * SWT_FIELD];
+      A.Uout[3 * NN + n] = s[S_M * SWT_FIELD];
+      if (nc == 4) A.Uout[4 * NN + n] = s[(S_U + 3) * SWT_FIELD];
     }
   }
   __syncthreads();  // the tile is reused by the block's next work item
