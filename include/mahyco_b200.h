@@ -295,9 +295,10 @@ int mhc_batch_set_grid_scale(mhc_batch* b, int scale);
  * back to the batch-wide value); the autotuner sets these */
 int mhc_batch_set_stage_grid_scale(mhc_batch* b, int stage, int scale);
 /* layout of the y / z remap sweeps of classical-limiter cases, for cells
- * and for nodes: 0 = by mesh size (default), 1 = one warp per line,
- * 2 = shared-memory tile, 3 = one thread per line chunk.  Results are the
- * same bit for bit whatever the layout; the autotuner picks the fastest.
+ * and for nodes: 0 = the default (the tile), 1 = one warp per line,
+ * 2 = shared-memory tile, 3 = the tile too (once one thread per line chunk).
+ * Results are the same bit for bit whatever the layout; the autotuner picks
+ * the fastest.
  * The _case_ variants set them, and the per-phase grid scale, for one case
  * run alone. */
 int mhc_batch_set_sweep_layout(mhc_batch* b, int cell_layout, int node_layout);

@@ -326,7 +326,7 @@ class Hydro:
 
     # IEquationOfState (src/eos/IEquationOfState.h:38-65), per environment
     def set_sweep_layout(self, cell_layout: int, node_layout: int):
-        """y / z sweep layouts: 0 by mesh size, 1 warp per line, 2 tile, 3 line chunks."""
+        """y / z sweep layouts: 1 warp per line; 0 (default), 2 and 3 the shared-memory tile."""
         _check(self.lib, self.lib.mhc_case_set_sweep_layout(self.h, int(cell_layout), int(node_layout)),
                "sweep layout")
 
@@ -472,7 +472,7 @@ class Batch:
         _check(self.lib, self.lib.mhc_batch_set_grid_scale(self.b, int(scale)), "grid scale")
 
     def set_sweep_layout(self, cell_layout: int, node_layout: int):
-        """y / z sweep layouts: 0 by mesh size, 1 warp per line, 2 tile, 3 line chunks."""
+        """y / z sweep layouts: 1 warp per line; 0 (default), 2 and 3 the shared-memory tile."""
         _check(self.lib, self.lib.mhc_batch_set_sweep_layout(self.b, int(cell_layout), int(node_layout)),
                "sweep layout")
 

@@ -5,12 +5,10 @@ arithmetic, so the tuning cycles are ordinary cycles of the run and the
 results are bit-identical whatever the tuner picks:
 
 * the layout of the y / z remap sweeps of classical-limiter cases, for
-  cells and for nodes: one warp per line (lanes along the sweep), a
+  cells and for nodes: one warp per line (lanes along the sweep) or a
   shared-memory tile (coalesced row loads, the warp-per-line arithmetic on
-  staged values) or one thread per line chunk (lanes along x, the stencil
-  carried in registers).  Which wins depends on the mesh size and the
-  number of environments (line chunks per sweep against the device's
-  thread slots);
+  staged values); layout 3, once one thread per line chunk, is the tile
+  again;
 * the grid of every phase's work-list launch: 0 launches one block per work
   item and lets the hardware balance them, k > 0 launches k times the blocks
   the device holds at once, persistent blocks striding over the list (the
@@ -23,9 +21,9 @@ log2(cells) -- in a JSON cache (MHC_TUNE_CACHE, default
 ~/.cache/mahyco_b200/tune.json), so the next run of the same bucket installs
 them without measuring.
 
-The tile width, the warps per block of the warp-per-line sweeps and the
-line-chunk length are template constants of the kernels, fixed at build time
-by measurement (mhc_sweep.cuh); the tuner chooses among the compiled layouts.
+The tile width and the warps per block of the warp-per-line sweeps are
+template constants of the kernels, fixed at build time by measurement
+(mhc_sweep.cuh); the tuner chooses among the compiled layouts.
 """
 from __future__ import annotations
 
@@ -34,7 +32,7 @@ import math
 import os
 
 CANDIDATES = (0, 1, 2, 4, 8)
-LAYOUTS = {1: "warp-per-line", 2: "tile", 3: "line-chunk"}
+LAYOUTS = {1: "warp-per-line", 2: "tile", 3: "tile (3)"}
 
 
 def cache_path() -> str:

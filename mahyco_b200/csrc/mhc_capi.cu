@@ -94,7 +94,7 @@ int engine_rebuild(Engine* e) {
     desc[i].P = h->d_params;
   }
   // groups
-  std::map<std::tuple<int, int, int, int, int, int, int, int, int, int, int, int, int, int, int, int>, int> gidx;
+  std::map<std::tuple<int, int, int, int, int, int, int, int, int, int, int, int, int, int>, int> gidx;
   std::vector<Group> old_groups;
   old_groups.swap(e->groups);
   for (int i = 0; i < nc; ++i) {
@@ -105,18 +105,16 @@ int engine_rebuild(Engine* e) {
     int sens = (int)((h->it_host - 1) % h->DIM);
     const int el = case_elasto(h) ? 1 : 0, hg = case_hourglass(h) ? 1 : 0;
     const int lim = node_sweep_mode(h->P), clim = cell_sweep_mode(h->P);
-    int cols, tile, ncols, ntile;
-    sweep_masks(h, e->cell_layout, false, cols, tile);
-    sweep_masks(h, e->node_layout, true, ncols, ntile);
+    const int tile = tile_mask(h, e->cell_layout, false), ntile = tile_mask(h, e->node_layout, true);
     const int cbc = case_cell_bcs(h) ? 1 : 0;
     const int adv = h->P.sans_lagrange ? 1 : 0, csts = (h->P.schema_csts && h->P.with_projection) ? 1 : 0;
-    auto key = std::make_tuple(h->DIM, h->NE, euler, skip_mask(h), sens, el, hg, lim, clim, cols, ncols, cbc, tile, ntile,
+    auto key = std::make_tuple(h->DIM, h->NE, euler, skip_mask(h), sens, el, hg, lim, clim, cbc, tile, ntile,
                                adv, csts);
     auto it = gidx.find(key);
     if (it == gidx.end()) {
       Group g;
       g.DIM = h->DIM; g.NE = h->NE; g.EULER = euler; g.skip = skip_mask(h); g.it0 = h->it_host;
-      g.EL = el; g.HG = hg; g.LIM = lim; g.CLIM = clim; g.COLS = cols; g.NCOLS = ncols; g.CBC = cbc; g.TILE = tile; g.NTILE = ntile;
+      g.EL = el; g.HG = hg; g.LIM = lim; g.CLIM = clim; g.CBC = cbc; g.TILE = tile; g.NTILE = ntile;
       g.ADV = adv;
       g.CSTS = csts;
       gidx[key] = (int)e->groups.size();
@@ -153,8 +151,8 @@ int engine_rebuild(Engine* e) {
               phase(g.fin_cells, PH_CELLS) && phase(g.fin_nodes, PH_NODES) && phase(g.dt, PH_CELLS) &&
               phase(g.lag_nodes, PH_NODES);
     for (int D = 0; D < g.DIM; ++D)
-      ok = ok && phase(g.sw_cells[D], group_cell_phase(g.CLIM, g.COLS, g.TILE, D)) &&
-           phase(g.sw_nodes[D], group_node_phase(g.LIM, g.NCOLS, g.NTILE, D));
+      ok = ok && phase(g.sw_cells[D], group_cell_phase(g.CLIM, g.TILE, D)) &&
+           phase(g.sw_nodes[D], group_node_phase(g.LIM, g.NTILE, D));
     if (!ok) return set_err(MHC_ERR_ARG, "more than 2^31 blocks in one phase of a batch");
   }
   // the same cases again (HydroStartInit on a case that ran): the lists are

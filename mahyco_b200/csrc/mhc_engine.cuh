@@ -76,10 +76,8 @@ struct Group {
   int CBC = 0;                 // cell-variable boundary conditions (Density, Energy, Pressure)
   int LIM = 0;                 // node-sweep instance: limiter 0-2, LIM_ORDER1 or LIM_GEN
   int CLIM = 0;                // cell-sweep instance: the same, LIM_O3 (third order) or LIM_PB (pente-borne)
-  int COLS = 0;                // bit D: the classical cell sweep along D uses one thread per line chunk
-  int TILE = 0;                // bit D: ... or a shared-memory tile (when not COLS)
-  int NTILE = 0;               // bit D: the node sweep along D uses a shared-memory tile (when not NCOLS)
-  int NCOLS = 0;               // bit D: the same for the node sweep
+  int TILE = 0;                // bit D: the classical cell sweep along D goes through a shared-memory tile
+  int NTILE = 0;               // bit D: the same for the node sweep
   int ADV = 0;                 // sans-lagrange: prescribed velocities, no Lagrange phase, no dual projection
   int CSTS = 0;                // schema-csts with the remap: half-step velocity updates around the step
   int CET = 0;                 // a member has conservation-energie-totale (finalize cells reads the dual variables)
@@ -89,8 +87,8 @@ struct Group {
   // and the phase of the sweep rotation
   bool same_launches(const Group& o) const {
     return DIM == o.DIM && NE == o.NE && EULER == o.EULER && skip == o.skip && EL == o.EL && HG == o.HG &&
-           CBC == o.CBC && LIM == o.LIM && CLIM == o.CLIM && COLS == o.COLS && TILE == o.TILE && NTILE == o.NTILE &&
-           NCOLS == o.NCOLS && ADV == o.ADV && CSTS == o.CSTS && CET == o.CET && it0 % 6 == o.it0 % 6 &&
+           CBC == o.CBC && LIM == o.LIM && CLIM == o.CLIM && TILE == o.TILE && NTILE == o.NTILE &&
+           ADV == o.ADV && CSTS == o.CSTS && CET == o.CET && it0 % 6 == o.it0 % 6 &&
            members == o.members;
   }
   DevList init_cells, init_nodes, lag_nodes, lag_cells, fin_cells, fin_nodes, dt;
@@ -134,8 +132,8 @@ struct Engine {
   bool side_failed = false;
   int forked = 0;  // sweeps of this remap whose node sweeps are on the side stream, not joined yet
   // layout of the y / z sweeps of classical-limiter cases, set by a caller
-  // or the tuner (mhc_*_set_sweep_layout): 0 = by mesh size (the line-chunk
-  // thresholds), 1 = warp per line, 2 = shared-memory tile, 3 = line chunks
+  // or the tuner (mhc_*_set_sweep_layout): 1 = warp per line, 0, 2 and 3 =
+  // shared-memory tile
   int cell_layout = 0, node_layout = 0;
   // kernels this engine put on the GPU (graph replays count their nodes)
   long long launches = 0;
@@ -236,99 +234,27 @@ inline int cell_sweep_mode(const mhc_case_params& P) {
   return P.ordre_projection == 3 ? LIM_O3 : node_sweep_mode(P);
 }
 
-// Directions whose classical cell sweep runs one thread per line chunk
-// (body_sweep_cells_cols): coalesced but with one line chunk per thread, it
-// pays when the sweep has enough line chunks to fill the device many times
-// over (large meshes); smaller meshes keep the warp-per-line layout.  The
-// node sweep, with fewer registers per line, pays from a quarter of that.
-// The thresholds (line chunks of the sweep) can be changed with the
-// environment variables MHC_SWEEP_COLS_MIN_THREADS (cells) and
-// MHC_SWEEP_NODE_COLS_MIN_THREADS (nodes; default: the cell threshold / 4),
-// read when the launch lists are built (0: every y / z sweep in this layout).
-inline long long cols_min_threads() {
-  const char* s = getenv("MHC_SWEEP_COLS_MIN_THREADS");
-  if (s && *s) return atoll(s);
-  return 1LL << 18;
-}
-inline long long node_cols_min_threads() {
-  const char* s = getenv("MHC_SWEEP_NODE_COLS_MIN_THREADS");
-  if (s && *s) return atoll(s);
-  return cols_min_threads() / 4;
-}
-inline int cols_mask(const mhc_case* h) {
-  if (cell_sweep_mode(h->P) > LIM_ORDER1) return 0;
-  const long long lim = cols_min_threads();
-  int m = 0;
-  for (int D = 1; D < h->DIM; ++D) {
-    const int nd = D == 1 ? h->M.ncy : h->M.ncz, nb = D == 1 ? h->M.ncz : h->M.ncy;
-    if ((long long)h->M.ncx * nb * col_chunks(nd) >= lim) m |= 1 << D;
-  }
-  return m;
-}
-inline int node_cols_mask(const mhc_case* h) {
-  if (node_sweep_mode(h->P) > LIM_ORDER1) return 0;
-  const long long lim = node_cols_min_threads();
-  int m = 0;
-  for (int D = 1; D < h->DIM; ++D) {
-    const int nd = D == 1 ? h->M.nny : h->M.nnz, nb = D == 1 ? h->M.nnz : h->M.nny;
-    if ((long long)h->M.nnx * nb * col_chunks(nd) >= lim) m |= 1 << D;
-  }
-  return m;
-}
-
-// Directions whose classical cell sweep goes through a shared-memory tile
-// (body_sweep_cells_tile: coalesced loads and stores, the warp-per-line
-// arithmetic): every y / z sweep that does not take the line-chunk layout.
-// MHC_SWEEP_TILE=0 in the environment keeps the warp-per-line layout.
-inline int tile_mask(const mhc_case* h) {
-  if (cell_sweep_mode(h->P) > LIM_ORDER1) return 0;
+// Directions whose classical cell (nodes: node) sweep goes through a
+// shared-memory tile (body_sweep_cells_tile: coalesced loads and stores, the
+// warp-per-line arithmetic): every y / z sweep, unless the engine's layout is
+// 1 (warp per line) or MHC_SWEEP_TILE=0 is in the environment.  Layout 3, once
+// one thread per line chunk, is the tile too.
+inline int tile_mask(const mhc_case* h, int layout, bool nodes) {
+  // the seven elasto variables ride through the warp-per-line cell sweeps only
+  if (!nodes && h->P.env[0].elasto_model && h->P.with_projection) return 0;
+  if ((nodes ? node_sweep_mode(h->P) : cell_sweep_mode(h->P)) > LIM_ORDER1) return 0;
   const char* s = getenv("MHC_SWEEP_TILE");
-  if (s && *s == '0') return 0;
-  int m = 0;
-  for (int D = 1; D < h->DIM; ++D) m |= 1 << D;
-  return m & ~cols_mask(h);
+  if (layout == 1 || (layout == 0 && s && *s == '0')) return 0;
+  return h->DIM == 3 ? 6 : 2;
 }
 
-// the same for the node sweeps (MHC_SWEEP_TILE=0 also keeps their
-// warp-per-line layout)
-inline int node_tile_mask(const mhc_case* h) {
-  if (node_sweep_mode(h->P) > LIM_ORDER1) return 0;
-  const char* s = getenv("MHC_SWEEP_TILE");
-  if (s && *s == '0') return 0;
-  int m = 0;
-  for (int D = 1; D < h->DIM; ++D) m |= 1 << D;
-  return m & ~node_cols_mask(h);
-}
-
-inline int group_node_phase(int LIM, int NCOLS, int NTILE, int D) {
-  if ((NCOLS >> D) & 1) return node_sweep_phase(LIM_COLS + LIM, D);
-  if ((NTILE >> D) & 1) return PH_SWNT0 + D;
-  return node_sweep_phase(LIM, D);
-}
-
-// the (line-chunk, tile) direction masks of a case's cell or node sweeps
-// under an engine's layout choice
-inline void sweep_masks(const mhc_case* h, int layout, bool nodes, int& cols, int& tile) {
-  if (!nodes && h->P.env[0].elasto_model && h->P.with_projection) {
-    // the seven elasto variables ride through the warp-per-line cell sweeps only
-    cols = tile = 0;
-    return;
-  }
-  cols = nodes ? node_cols_mask(h) : cols_mask(h);
-  tile = nodes ? node_tile_mask(h) : tile_mask(h);
-  const int mode = nodes ? node_sweep_mode(h->P) : cell_sweep_mode(h->P);
-  if (layout == 0 || mode > LIM_ORDER1) return;
-  int all = 0;
-  for (int D = 1; D < h->DIM; ++D) all |= 1 << D;
-  cols = layout == 3 ? all : 0;
-  tile = layout == 2 ? all : 0;
+inline int group_node_phase(int LIM, int NTILE, int D) {
+  return ((NTILE >> D) & 1) ? PH_SWNT0 + D : node_sweep_phase(LIM, D);
 }
 
 // phase of the cell sweep of a group along D
-inline int group_cell_phase(int CLIM, int COLS, int TILE, int D) {
-  if ((COLS >> D) & 1) return cell_sweep_phase(LIM_COLS + CLIM, D);
-  if ((TILE >> D) & 1) return PH_SWCT0 + D;
-  return cell_sweep_phase(CLIM, D);
+inline int group_cell_phase(int CLIM, int TILE, int D) {
+  return ((TILE >> D) & 1) ? PH_SWCT0 + D : cell_sweep_phase(CLIM, D);
 }
 
 // directions the remap does not sweep: one cell thick, or not the axis of a

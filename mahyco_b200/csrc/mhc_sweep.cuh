@@ -1073,136 +1073,6 @@ __device__ __forceinline__ void body_sweep_cells_o3(const Mesh& M, const Fields&
 }
 
 // ---------------------------------------------------------------------------
-// Cell sweep along D = 1, 2, classical limiters and first order, with one
-// thread per line: the threads of a warp hold consecutive x columns, so
-// every load and store is coalesced, and each thread walks a chunk of its
-// line in order with the stencil carried in registers.  Iteration q loads
-// cell q and the node plane in front of it; it completes the face gradient
-// of face q, the limited gradient of cell q-1, the value of face q-1 and the
-// update of cell q-2.  A chunk writes cells [o0, o1) and starts two cells
-// before o0.  Same arithmetic, in the same order, as
-// body_sweep_cells_lanes.
-// ---------------------------------------------------------------------------
-constexpr int SWC_CHUNK = 16;   // cells written per thread at most
-
-// chunks of a line of nd cells, and the cells [o0, o1) of chunk ch
-__host__ __device__ inline int col_chunks(int nd) { return (nd + SWC_CHUNK - 1) / SWC_CHUNK; }
-__host__ __device__ inline void col_chunk_range(int nd, int ch, int& o0, int& o1) {
-  const int n = col_chunks(nd);
-  const int len = (nd + n - 1) / n;
-  o0 = ch * len;
-  o1 = o0 + len < nd ? o0 + len : nd;
-}
-
-template <int DIM, int NE, int D, int LIM>
-__device__ __forceinline__ void body_sweep_cells_cols(const Mesh& M, const Fields& F, const SweepArgs& A, int vbx,
-                                                      int vby) {
-  static_assert(D >= 1, "x sweeps use the lane layout");
-  constexpr int NV = 3 * NE + 1;
-  constexpr int NQ = DIM == 3 ? 4 : 2;
-  const long long N = M.ncell;
-  const int nd = D == 1 ? M.ncy : M.ncz;
-  const int nb = D == 1 ? M.ncz : M.ncy;           // slow transverse extent
-  const long long col = (long long)vbx * SW_THREADS + threadIdx.x;
-  if (col >= (long long)M.ncx * nb) return;
-  const int tb = (int)((unsigned)col / (unsigned)M.ncx), i = (int)col - tb * M.ncx;
-  int o0, o1;
-  col_chunk_range(nd, vby, o0, o1);
-  if (o0 >= o1) return;
-  const double dt = F.s->dt;
-  const int order2 = LIM == LIM_ORDER1 ? 0 : 1;  // ordre-projection - 1
-  const double* __restrict__ Uin = A.Uin;
-  auto cell_at = [&](int p) -> long long { return D == 1 ? cell_id(M, i, p, tb) : cell_id(M, i, tb, p); };
-  auto plane_at = [&](int p, Plane<DIM>& P) {
-    if (D == 1) load_plane<DIM, D>(M, F, i, p, tb, P);
-    else load_plane<DIM, D>(M, F, i, tb, p, P);
-  };
-  // carried state: 1 = previous cell / face, 2 = the one before; lc = the
-  // upwind value of face q-1 taken from its back cell q-2 (made one
-  // iteration early, when that cell's limited gradient is known, so that
-  // neither the gradient nor phi of cell q-2 has to be carried)
-  double phi1[NV], gf1[NV], lc[NV], pf2[NV];
-  double xc1 = 0., xc2 = 0., fc1 = 0., un1 = 0., un2 = 0., L1 = 0., L2 = 0.;
-  const int qs = o0 - 2 > 0 ? o0 - 2 : 0;
-  Plane<DIM> cur;       // back plane of cell q
-  plane_at(qs, cur);
-#pragma unroll
-  for (int v = 0; v < NV; ++v) phi1[v] = gf1[v] = lc[v] = pf2[v] = 0.;
-  for (int q = qs; q <= o1 + 1; ++q) {
-    const bool cell = q < nd;                 // a cell is loaded at q
-    double phi[NV], xc = 0.;
-    Plane<DIM> nxt;
-    if (cell) {
-      plane_at(q + 1, nxt);
-      xc = centre_from_planes<DIM, D>(cur, nxt);
-      const long long c = cell_at(q);
-      double u[NV], den;
-#pragma unroll
-      for (int v = 0; v < NV; ++v) u[v] = __ldg(Uin + v * N + c);
-      if (A.first) {
-        den = __ldg(F.V + c);
-      } else {
-        den = 0.;
-#pragma unroll
-        for (int e = 0; e < NE; ++e) den += u[e];
-      }
-#pragma unroll
-      for (int v = 0; v < NV; ++v) phi[v] = div_rn(u[v], den);
-    } else {
-#pragma unroll
-      for (int v = 0; v < NV; ++v) phi[v] = 0.;
-    }
-    const bool face_q = cell && q > 0;        // face q (between q-1 and q) is inner
-    const double dx = xc - xc1;
-    const bool face_q1 = q - 1 > 0 && q - 1 < nd;  // face q-1 is inner
-    // face q-1 upwind test (its normal velocity and the centres of q-2, q-1)
-    const bool up_left = un1 * (xc1 - xc2) > 0.0;
-    double pf1[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const double gf = face_q ? div_rn(phi[v] - phi1[v], dx) : 0.;
-      // limited gradient of cell q-1 from its back (gf1) and front (gf) faces
-      const double gr1 = (LIM != LIM_ORDER1 && q - 1 >= 0 && q - 1 < nd) ? limited_gradient_t<LIM>(gf1[v], gf) : 0.;
-      pf1[v] = 0.;
-      if (face_q1) pf1[v] = up_left ? lc[v] : phi1[v] + order2 * (fc1 - xc1) * gr1;
-      // face q seen from its back cell q-1 (fc of face q = cur.fc)
-      lc[v] = phi1[v] + order2 * (cur.fc - xc1) * gr1;
-      gf1[v] = gf;
-    }
-    // update of cell o = q - 2 from faces o (pf2) and o + 1 (pf1)
-    const int o = q - 2;
-    if (o >= o0 && o < o1) {
-      const long long c = cell_at(o);
-      double ondB, ondF;
-      sweep_normals<DIM, D>(M, o, i, tb, ondB, ondF);
-      const bool fb = o > 0, ff = o + 1 < nd;
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        const double fB = fb ? ondB * un2 * L2 * dt * pf2[v] : 0.;
-        const double fF = ff ? ondF * un1 * L1 * dt * pf1[v] : 0.;
-        double sumf = 0., dual = 0.;
-        if (fb) { sumf += fB; dual += 0.5 * fB * ondB; }
-        if (ff) { sumf += fF; dual += 0.5 * fF * ondF; }
-        double uo = __ldg(Uin + v * N + c) - sumf;
-        if (v >= NE && v < 3 * NE && uo < 0.) uo = 0.;  // masses and energies stay >= 0
-        A.Uout[v * N + c] = uo;
-        if (v >= NE && v < 2 * NE) F.mflux[(v - NE) * N + c] = dual;
-      }
-    }
-    // shift
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      phi1[v] = phi[v];
-      pf2[v] = pf1[v];
-    }
-    xc2 = xc1; xc1 = xc;
-    un2 = un1; L2 = L1;
-    un1 = cur.un; L1 = cur.L; fc1 = cur.fc;
-    if (cell) cur = nxt;
-  }
-}
-
-// ---------------------------------------------------------------------------
 // Cell sweep along D = 1, 2 through a shared-memory tile, classical limiters
 // and first order.  A block holds SWT_COLS neighbouring x columns and one
 // window of 32 positions along D (the concatenated lines of the lane layout:
@@ -1218,6 +1088,10 @@ __device__ __forceinline__ void body_sweep_cells_cols(const Mesh& M, const Field
 //  3. Store: the load layout again, written cells only.
 // The staged front-plane coordinates of a cell are loaded, not shuffled, so
 // the cell centre is the same sum of the same node coordinates.
+//
+// For meshes of every size: a y or z sweep of 384^3 cells takes 2.3 ms here,
+// 2.6 ms with one thread per line chunk and the stencil carried in registers
+// (3 blocks per SM), 5.6 ms with a warp per line.
 // ---------------------------------------------------------------------------
 constexpr int SWT_COLS = 8;                     // x columns (warps) per block
 constexpr int SWT_THREADS = SWT_COLS * SW_LANES;
@@ -1554,164 +1428,6 @@ __device__ __forceinline__ void body_sweep_nodes_lanes(const Mesh& M, const Fiel
     if (out) A.Uout[4 * NN + n] = K.inner ? W : U;
   }
   if (out) A.Uout[3 * NN + n] = K.inner ? m + (K.bfm - K.ffm) : m;
-}
-
-// ---------------------------------------------------------------------------
-// Node sweep along D = 1, 2, classical limiters and first order, one thread
-// per line chunk (the layout of body_sweep_cells_cols).  Iteration q loads
-// node q; it completes the limited gradient of node q-1 and the update of
-// node q-2.  A chunk writes nodes [o0, o1) and starts two nodes before o0.
-// Same arithmetic, in the same order, as body_sweep_nodes_lanes.
-// ---------------------------------------------------------------------------
-// projected and phi values, position along D and front mass flux of node
-// (i, j, k) with index id along D
-// projected dual variables of node n before this sweep: the previous
-// sweep's output, or momentum, mass and kinetic energy from the node state
-__device__ __forceinline__ void node_u(const Fields& F, const DualArgs& A, long long NN, long long n, double (&U)[5]) {
-  if (A.Uin) {
-#pragma unroll
-    for (int q = 0; q < 5; ++q) U[q] = __ldg(A.Uin + q * NN + n);
-  } else {
-    const double mn = __ldg(F.mn + n), vx = __ldg(F.vx + n), vy = __ldg(F.vy + n), vz = __ldg(F.vz + n);
-    U[0] = mn * vx; U[1] = mn * vy; U[2] = mn * vz; U[3] = mn;
-    U[4] = 0.5 * mn * (vx * vx + vy * vy + vz * vz);
-  }
-}
-
-template <int DIM, int NE, int D>
-__device__ __forceinline__ void node_state(const Mesh& M, const Fields& F, const DualArgs& A, int i, int j, int k,
-                                           int id, double (&ph)[4], double& x, double& ffm) {
-  const long long NN = M.nnode, N = M.ncell;
-  const long long n = node_id(M, i, j, k);
-  x = __ldg(F.Xn[D] + n);
-  bool was_inner = false;
-#pragma unroll
-  for (int d = 0; d < DIM; ++d)
-    if (((A.done_dirs >> d) & 1) && node_inner_dir(M, i, j, k, d)) was_inner = true;
-  double U[5];
-  node_u(F, A, NN, n, U);
-  if (was_inner) {
-    ph[0] = div_rn(U[0], U[3]); ph[1] = div_rn(U[1], U[3]); ph[2] = div_rn(U[2], U[3]);
-    ph[3] = div_rn(U[4], U[3]);
-  } else {
-    const double vx = __ldg(F.vx + n), vy = __ldg(F.vy + n), vz = __ldg(F.vz + n);
-    ph[0] = vx; ph[1] = vy; ph[2] = vz;
-    ph[3] = 0.5 * (vx * vx + vy * vy + vz * vz);
-  }
-  ffm = 0.;
-  const int ndc = D == 1 ? M.ncy : M.ncz;
-  if (id < ndc) {
-    const double w = DIM == 2 ? .5 : .25;
-#pragma unroll
-    for (int b2 = 0; b2 < (DIM == 3 ? 2 : 1); ++b2) {
-#pragma unroll
-      for (int b1 = 0; b1 < 2; ++b1) {
-        int ci = i, cj = j, ck = k;
-        const int t1 = b1 - 1, t2 = b2 - 1;
-        if (D == 1) { ci += t1; ck += (DIM == 3 ? t2 : 0); }
-        else { ci += t1; cj += t2; }
-        if (ci < 0 || cj < 0 || ck < 0) continue;
-        if (ci >= M.ncx) continue;
-        if (D != 1 && cj >= M.ncy) continue;
-        if (DIM == 3 && D != 2 && ck >= M.ncz) continue;
-        const long long cf = cell_id(M, ci, cj, DIM == 3 ? ck : 0);
-#pragma unroll
-        for (int q = 0; q < NE; ++q) ffm += w * __ldg(F.mflux + q * N + cf);
-      }
-    }
-  }
-}
-
-template <int DIM, int NE, int D, int LIM>
-__device__ __forceinline__ void body_sweep_nodes_cols(const Mesh& M, const Fields& F, const DualArgs& A, int vbx,
-                                                      int vby) {
-  static_assert(D >= 1, "x sweeps use the lane layout");
-  const long long NN = M.nnode;
-  const int nn = D == 1 ? M.nny : M.nnz;
-  const int nb = D == 1 ? M.nnz : M.nny;
-  const long long col = (long long)vbx * SW_THREADS + threadIdx.x;
-  if (col >= (long long)M.nnx * nb) return;
-  const int tb = (int)((unsigned)col / (unsigned)M.nnx), i = (int)col - tb * M.nnx;
-  int o0, o1;
-  col_chunk_range(nn, vby, o0, o1);
-  if (o0 >= o1) return;
-  const double dt = F.s->dt;
-  const int order2 = LIM == LIM_ORDER1 ? 0 : A.order - 1;  // ordre-projection - 1
-  // carried state: 1 = node q-1, 2 = node q-2, 3 = node q-3
-  // fd1: forward difference of node q-2 (= backward difference of q-1);
-  // the projected variables of the node being updated are read again
-  // (cached) rather than carried, to keep registers for resident warps
-  double ph1[4], ph2[4], ph3[4], g1[3], g2[3], g3[3], fd1[3];
-  double x1 = 0., x2 = 0., x3 = 0., ffm1 = 0., ffm2 = 0., ffm3 = 0.;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) ph1[q] = ph2[q] = ph3[q] = 0.;
-#pragma unroll
-  for (int q = 0; q < 3; ++q) g1[q] = g2[q] = g3[q] = fd1[q] = 0.;
-  const int qs = o0 - 2 > 0 ? o0 - 2 : 0;
-  for (int q = qs; q <= o1 + 1; ++q) {
-    double ph[4] = {0., 0., 0., 0.}, x = 0., ffm = 0.;
-    if (q < nn) {
-      if (D == 1) node_state<DIM, NE, D>(M, F, A, i, q, tb, q, ph, x, ffm);
-      else node_state<DIM, NE, D>(M, F, A, i, tb, q, q, ph, x, ffm);
-    }
-    // limited gradients of node q-1 (inner nodes only); its backward
-    // difference is the forward difference of node q-2, carried from the
-    // previous iteration (valid from the second iteration on, the first
-    // node whose gradient an update needs)
-    const int m = q - 1;
-    double gm[3], fd[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      gm[c] = 0.;
-      fd[c] = LIM != LIM_ORDER1 ? div_rn(ph[c] - ph1[c], x - x1) : 0.;
-      if (LIM != LIM_ORDER1 && m > 0 && m < nn - 1) gm[c] = limited_gradient_t<LIM>(fd1[c], fd[c]);
-    }
-    // update of node o = q - 2: neighbours o-1 (3), o (2), o+1 (1)
-    const int o = q - 2;
-    if (o >= o0 && o < o1) {
-      const long long n = D == 1 ? node_id(M, i, o, tb) : node_id(M, i, tb, o);
-      double V[5];
-      node_u(F, A, NN, n, V);
-      if (o > 0 && o < nn - 1) {
-        const double bfm = ffm3, ffm_o = ffm2;
-        V[3] += bfm - ffm_o;
-        double FV[3], BV[3], FE, BE;
-        {
-          const double ufront = 0.5 * (ph2[D] + ph1[D]);
-          const int signfront = (ufront > 0) ? 1 : -1;
-          const bool fr = ffm_o < 0.;
-          const double geo = (signfront * (x1 - x2) - dt * ufront);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) FV[c] = (fr ? ph1[c] : ph2[c]) + order2 * (0.5 * (fr ? gm[c] : g1[c]) * geo);
-          FE = (fr ? ph1[3] : ph2[3]) + order2 * (0.5 * 0. * geo);
-        }
-        {
-          const double uback = 0.5 * (ph3[D] + ph2[D]);
-          const int signback = (uback > 0) ? 1 : -1;
-          const bool bk = bfm > 0.;
-          const double geo = (signback * (x2 - x3) - dt * uback);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) BV[c] = (bk ? ph3[c] : ph2[c]) + order2 * (0.5 * (bk ? g2[c] : g1[c]) * geo);
-          BE = (bk ? ph3[3] : ph2[3]) + order2 * (0.5 * 0. * geo);
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) V[c] += bfm * BV[c] - ffm_o * FV[c];
-        V[4] += bfm * BE - ffm_o * FE;
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          if (fabs(V[c]) < 1.e-300) V[c] = 0.;
-      }
-#pragma unroll
-      for (int c = 0; c < 5; ++c) A.Uout[c * NN + n] = V[c];
-    }
-    // shift
-#pragma unroll
-    for (int c = 0; c < 4; ++c) { ph3[c] = ph2[c]; ph2[c] = ph1[c]; ph1[c] = ph[c]; }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) { g3[c] = g2[c]; g2[c] = g1[c]; g1[c] = gm[c]; fd1[c] = fd[c]; }
-    x3 = x2; x2 = x1; x1 = x;
-    ffm3 = ffm2; ffm2 = ffm1; ffm1 = ffm;
-  }
 }
 
 // ---------------------------------------------------------------------------

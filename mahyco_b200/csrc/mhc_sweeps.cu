@@ -21,13 +21,11 @@ void cell_sweep_elasto(Engine* e, Group& g, int D, int k) {
   else if constexpr (DIM == 3) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, 1, 2, LIM, MHC_ELASTO_XV, SOLO>), SW_THREADS, 0, g.sw_cells[2], k);
 }
 
-// (no line chunks along x: every mask of such a layout is over D = 1, 2)
 template <int DIM, int NE, int LIM>
 void cell_sweep(Engine* e, Group& g, int D, int k) {
   StageTimer tm(e, MHC_STAGE_SWEEP_CELLS);
-  if (D == 0) {
-    if constexpr (LIM < LIM_COLS) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 0, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[0], k);
-  } else if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 1, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[1], k);
+  if (D == 0) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 0, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[0], k);
+  else if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 1, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[1], k);
   else if constexpr (DIM == 3) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 2, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[2], k);
 }
 
@@ -50,9 +48,8 @@ void node_sweep_tile(Engine* e, Group& g, int D, int k) {
 template <int DIM, int NE, int LIM>
 void node_sweep(Engine* e, Group& g, int D, int k) {
   StageTimer tm(e, MHC_STAGE_SWEEP_NODES);
-  if (D == 0) {
-    if constexpr (LIM < LIM_COLS) plaunch_case(e, MHC_KERNEL(kb_sweep_nodes<DIM, NE, 0, LIM, SOLO>), SW_THREADS, 0, g.sw_nodes[0], k);
-  } else if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_nodes<DIM, NE, 1, LIM, SOLO>), SW_THREADS, 0, g.sw_nodes[1], k);
+  if (D == 0) plaunch_case(e, MHC_KERNEL(kb_sweep_nodes<DIM, NE, 0, LIM, SOLO>), SW_THREADS, 0, g.sw_nodes[0], k);
+  else if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_nodes<DIM, NE, 1, LIM, SOLO>), SW_THREADS, 0, g.sw_nodes[1], k);
   else if constexpr (DIM == 3) plaunch_case(e, MHC_KERNEL(kb_sweep_nodes<DIM, NE, 2, LIM, SOLO>), SW_THREADS, 0, g.sw_nodes[2], k);
 }
 
@@ -61,7 +58,6 @@ void node_sweep(Engine* e, Group& g, int D, int k) {
 // one direction of the remap for a group: cell sweep, then node sweep
 template <int DIM, int NE>
 void sweep_step_dn(Engine* e, Group& g, int D, int k) {
-  const int cl = ((g.COLS >> D) & 1) ? LIM_COLS + g.CLIM : g.CLIM;
   side_reuse(e, k);
   if (NE == 1 && g.EL && g.EULER) {
     if constexpr (NE == 1) {
@@ -72,18 +68,14 @@ void sweep_step_dn(Engine* e, Group& g, int D, int k) {
         default: cell_sweep_elasto<DIM, LIM_ORDER1>(e, g, D, k); break;
       }
     }
-  } else if (D > 0 && !((g.COLS >> D) & 1) && ((g.TILE >> D) & 1)) {
+  } else if (D > 0 && ((g.TILE >> D) & 1)) {
     switch (g.CLIM) {
       case 0: cell_sweep_tile<DIM, NE, 0>(e, g, D, k); break;
       case 1: cell_sweep_tile<DIM, NE, 1>(e, g, D, k); break;
       case 2: cell_sweep_tile<DIM, NE, 2>(e, g, D, k); break;
       default: cell_sweep_tile<DIM, NE, LIM_ORDER1>(e, g, D, k); break;
     }
-  } else switch (cl) {
-    case LIM_COLS + 0: cell_sweep<DIM, NE, LIM_COLS + 0>(e, g, D, k); break;
-    case LIM_COLS + 1: cell_sweep<DIM, NE, LIM_COLS + 1>(e, g, D, k); break;
-    case LIM_COLS + 2: cell_sweep<DIM, NE, LIM_COLS + 2>(e, g, D, k); break;
-    case LIM_COLS + LIM_ORDER1: cell_sweep<DIM, NE, LIM_COLS + LIM_ORDER1>(e, g, D, k); break;
+  } else switch (g.CLIM) {
     case 0: cell_sweep<DIM, NE, 0>(e, g, D, k); break;
     case 1: cell_sweep<DIM, NE, 1>(e, g, D, k); break;
     case 2: cell_sweep<DIM, NE, 2>(e, g, D, k); break;
@@ -94,19 +86,14 @@ void sweep_step_dn(Engine* e, Group& g, int D, int k) {
   }
   if (g.ADV) return;  // sans-lagrange: no dual projection (PrepareRemap.cc:211)
   NodeFork fork(e, k);
-  const int nl = ((g.NCOLS >> D) & 1) ? LIM_COLS + g.LIM : g.LIM;
-  if (D > 0 && !((g.NCOLS >> D) & 1) && ((g.NTILE >> D) & 1)) {
+  if (D > 0 && ((g.NTILE >> D) & 1)) {
     switch (g.LIM) {
       case 0: node_sweep_tile<DIM, NE, 0>(e, g, D, k); break;
       case 1: node_sweep_tile<DIM, NE, 1>(e, g, D, k); break;
       case 2: node_sweep_tile<DIM, NE, 2>(e, g, D, k); break;
       default: node_sweep_tile<DIM, NE, LIM_ORDER1>(e, g, D, k); break;
     }
-  } else switch (nl) {
-    case LIM_COLS + 0: node_sweep<DIM, NE, LIM_COLS + 0>(e, g, D, k); break;
-    case LIM_COLS + 1: node_sweep<DIM, NE, LIM_COLS + 1>(e, g, D, k); break;
-    case LIM_COLS + 2: node_sweep<DIM, NE, LIM_COLS + 2>(e, g, D, k); break;
-    case LIM_COLS + LIM_ORDER1: node_sweep<DIM, NE, LIM_COLS + LIM_ORDER1>(e, g, D, k); break;
+  } else switch (g.LIM) {
     case 0: node_sweep<DIM, NE, 0>(e, g, D, k); break;
     case 1: node_sweep<DIM, NE, 1>(e, g, D, k); break;
     case 2: node_sweep<DIM, NE, 2>(e, g, D, k); break;
