@@ -218,41 +218,67 @@ int rider_upload(mhc_case* h, cudaStream_t st) {
   const long long NN = M.nnode;
   const double Pi = 3.14159265359;
   const int kind = (P.cas_test - MHC_TEST_MONO_RIDER_TX) % 8;  // Tx Ty T45 Rotation Vortex Deformation (+2 reverse)
-  std::vector<double> v(3 * NN, 0.0);
-  for (long long n = 0; n < NN; ++n) {
-    const long long i = n % M.nnx, r = n / M.nnx, j = r % M.nny, k = r / M.nny;
-    const double x = M.o[0] + i * M.h[0], y = M.o[1] + j * M.h[1], z = M.dim == 3 ? M.o[2] + k * M.h[2] : 0.;
-    (void)z;
-    double vx = 0.0, vy = 0.0;
-    if (kind == 0) vx = 1.;
-    if (kind == 1) vy = 1.;
-    if (kind == 2) { vx = 1.0; vy = 1.0; }
-    if (kind == 3) {
-      const double ddx = x - 0.5, ddy = y - 0.5;
-      const double theta = std::atan2(ddy, ddx);
-      const double rr = std::sqrt(ddx * ddx + ddy * ddy);
-      const double omega = 4. * Pi;
-      vx = -rr * omega * std::sin(omega * 0. + theta);
-      vy = rr * omega * std::cos(omega * 0. + theta);
+  // The vortex and deformation fields are products of functions of x and of y:
+  // those are evaluated once per node line, not once per node, and the
+  // products formed in the reference's order.  The fields do not depend on z:
+  // one layer of nodes, then its copies.
+  const long long layer = (long long)M.nnx * M.nny;
+  std::vector<double> v(3 * NN, 0.0), fx(2 * M.nnx), fy(2 * M.nny);
+  auto X = [&](long long i) { return M.o[0] + i * M.h[0]; };
+  auto Y = [&](long long j) { return M.o[1] + j * M.h[1]; };
+  const bool vortex = kind == 4 || kind == 6, deformation = kind == 5 || kind == 7;
+  if (vortex || deformation) {
+    for (int i = 0; i < M.nnx; ++i) {
+      const double a = vortex ? Pi * X(i) : 4. * Pi * (X(i) + 0.5);
+      fx[2 * i] = std::cos(a);
+      fx[2 * i + 1] = std::sin(a);
     }
-    if (kind == 4 || kind == 6) {
-      vx = -2. * std::cos(Pi * y) * std::sin(Pi * y) * std::sin(Pi * x) * std::sin(Pi * x);
-      vy = 2. * std::cos(Pi * x) * std::sin(Pi * x) * std::sin(Pi * y) * std::sin(Pi * y);
+    for (int j = 0; j < M.nny; ++j) {
+      const double a = vortex ? Pi * Y(j) : 4. * Pi * (Y(j) + 0.5);
+      fy[2 * j] = std::cos(a);
+      fy[2 * j + 1] = std::sin(a);
     }
-    if (kind == 5 || kind == 7) {
-      const double ddx = x + 0.5, ddy = y + 0.5;
-      vx = std::sin(4. * Pi * ddx) * std::sin(4. * Pi * ddy);
-      vy = std::cos(4. * Pi * ddx) * std::cos(4. * Pi * ddy);
-    }
-    v[n] = vx;
-    v[NN + n] = vy;
   }
-  // pageable sources: each copy is staged before the call returns
+  for (int j = 0; j < M.nny; ++j) {
+    const double cy = fy[2 * j], sy = fy[2 * j + 1];
+    for (int i = 0; i < M.nnx; ++i) {
+      const double cx = fx[2 * i], sx = fx[2 * i + 1];
+      double vx = 0.0, vy = 0.0;
+      if (kind == 0) vx = 1.;
+      if (kind == 1) vy = 1.;
+      if (kind == 2) { vx = 1.0; vy = 1.0; }
+      if (kind == 3) {
+        const double ddx = X(i) - 0.5, ddy = Y(j) - 0.5;
+        const double theta = std::atan2(ddy, ddx);
+        const double rr = std::sqrt(ddx * ddx + ddy * ddy);
+        const double omega = 4. * Pi;
+        vx = -rr * omega * std::sin(omega * 0. + theta);
+        vy = rr * omega * std::cos(omega * 0. + theta);
+      }
+      if (vortex) {
+        vx = -2. * cy * sy * sx * sx;
+        vy = 2. * cx * sx * sy * sy;
+      }
+      if (deformation) {
+        vx = sx * sy;
+        vy = cx * cy;
+      }
+      const long long n = i + (long long)M.nnx * j;
+      v[n] = vx;
+      v[NN + n] = vy;
+    }
+  }
+  for (int k = 1; k < M.nnz; ++k)
+    for (int q = 0; q < 2; ++q) memcpy(&v[q * NN + k * layer], &v[q * NN], layer * sizeof(double));
+  // (a pageable source is staged before the call returns)
   const size_t b = NN * sizeof(double);
-  CK(cudaMemcpyAsync(h->F.vx, v.data(), b, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(h->F.vy, v.data() + NN, b, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(h->F.vz, v.data() + 2 * NN, b, cudaMemcpyHostToDevice, st));
-  if (h->F.v0) CK(cudaMemcpyAsync(h->F.v0, v.data(), 3 * b, cudaMemcpyHostToDevice, st));
+  double* const dev[3] = {h->F.vx, h->F.vy, h->F.vz};
+  if (h->F.v0) {
+    CK(cudaMemcpyAsync(h->F.v0, v.data(), 3 * b, cudaMemcpyHostToDevice, st));
+    for (int q = 0; q < 3; ++q) CK(cudaMemcpyAsync(dev[q], h->F.v0 + q * NN, b, cudaMemcpyDeviceToDevice, st));
+  } else {
+    for (int q = 0; q < 3; ++q) CK(cudaMemcpyAsync(dev[q], v.data() + q * NN, b, cudaMemcpyHostToDevice, st));
+  }
   return MHC_OK;
 }
 
