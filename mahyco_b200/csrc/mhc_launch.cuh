@@ -235,9 +235,11 @@ __global__ void __launch_bounds__(CT, MHC_NODES_MIN_BLOCKS) kb_lagrange_nodes(co
   }
 }
 
-// resident blocks per SM asked of the compiler for the geometry pass
+// resident blocks per SM asked of the compiler for the geometry pass: 4 (128
+// registers, 152 bytes of spills) against 3 (166, none) and 5 (96, 360 bytes):
+// 3.88, 3.98 and 5.14 ms at 384^3
 #ifndef MHC_GEOM_MIN_BLOCKS
-#define MHC_GEOM_MIN_BLOCKS 2
+#define MHC_GEOM_MIN_BLOCKS 4
 #endif
 
 template <int DIM, bool SOLO = false>
