@@ -215,6 +215,12 @@ __global__ void __launch_bounds__(CT) kb_init_nodes(const CaseDesc* __restrict__
 #ifndef MHC_LAG_MIN_BLOCKS
 #define MHC_LAG_MIN_BLOCKS 6
 #endif
+// with the geometry in the pass (elasto-plastic, CSTS) 3 (168 registers): the
+// spills of 80 registers, 600 bytes in 2D and 3 kB in 3D, cost more (bar
+// 80x400: 14.8 -> 13.6 us)
+#ifndef MHC_LAG_MIN_BLOCKS_GEO
+#define MHC_LAG_MIN_BLOCKS_GEO 3
+#endif
 
 // resident blocks per SM asked of the compiler for the node pass (a latency
 // bound gather: more warps in flight hide more of it)
@@ -260,7 +266,7 @@ __global__ void __launch_bounds__(CT, MHC_GEOM_MIN_BLOCKS) kb_lagrange_geom(cons
 // one more kernel for the scalars took 6.4 of the 21.0 us of an iteration on
 // 200 x 10 cells.  The entry points called one by one keep kb_delta_t.
 template <int DIM, int NE, bool EULER, bool EL, bool CSTS = false, bool DT = false, bool SOLO = false>
-__global__ void __launch_bounds__(CT, MHC_LAG_MIN_BLOCKS) kb_lagrange_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant__ PhaseList L) {
+__global__ void __launch_bounds__(CT, EL || CSTS ? MHC_LAG_MIN_BLOCKS_GEO : MHC_LAG_MIN_BLOCKS) kb_lagrange_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant__ PhaseList L) {
   MHC_FOR_ITEMS(L) {
     const WorkItem wi = item_at<PH_CELLS>(C, L, w_);
     Fields F = C.at(wi.c).F;
@@ -313,8 +319,18 @@ __global__ void __launch_bounds__(CT) kb_hourglass(const __grid_constant__ CaseT
 
 // the generalised-limiter and third-order instances hold more state per
 // lane and are asked for fewer resident blocks
+// the third-order sweep: 5 (96 registers; 101x37x35 cells 44 us at 4, 40 at 5);
+// the pente-borne one: 4 (128 registers; 350x150 cells, three environments: 35
+// us, 5 blocks 38 there and 6 % faster at 1200x500)
+#ifndef MHC_SW_MIN_BLOCKS_O3
+#define MHC_SW_MIN_BLOCKS_O3 5
+#endif
+#ifndef MHC_SW_MIN_BLOCKS_PB
+#define MHC_SW_MIN_BLOCKS_PB 4
+#endif
 template <int DIM, int NE, int D, int LIM, int XV = 0, bool SOLO = false>
-__global__ void __launch_bounds__(SW_THREADS, LIM >= LIM_GEN ? 2 : MHC_SW_MIN_BLOCKS_CELLS)
+__global__ void __launch_bounds__(SW_THREADS, LIM == LIM_PB ? MHC_SW_MIN_BLOCKS_PB
+                                              : (LIM == LIM_O3 ? MHC_SW_MIN_BLOCKS_O3 : (LIM == LIM_GEN ? 2 : MHC_SW_MIN_BLOCKS_CELLS)))
 kb_sweep_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant__ PhaseList L, int k) {
   MHC_FOR_ITEMS(L) {
     const WorkItem wi = item_at<cell_sweep_phase(LIM, D)>(C, L, w_);
@@ -425,9 +441,14 @@ kb_sweep_nodes(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant_
 #ifndef MHC_FIN_MIN_BLOCKS
 #define MHC_FIN_MIN_BLOCKS 6
 #endif
+// three environments or more: 4 (128 registers, no spills; 500 bytes at 6):
+// 350x150 cells 14.1 -> 12.0 us, 1200x500 within 3 %
+#ifndef MHC_FIN_MIN_BLOCKS_3
+#define MHC_FIN_MIN_BLOCKS_3 4
+#endif
 
 template <int DIM, int NE, bool ADV = false, bool SOLO = false>
-__global__ void __launch_bounds__(CT, MHC_FIN_MIN_BLOCKS) kb_remap_finalize_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant__ PhaseList L, int K) {
+__global__ void __launch_bounds__(CT, NE > 2 ? MHC_FIN_MIN_BLOCKS_3 : MHC_FIN_MIN_BLOCKS) kb_remap_finalize_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant__ PhaseList L, int K) {
   MHC_FOR_ITEMS(L) {
     const WorkItem wi = item_at<PH_CELLS>(C, L, w_);
     Fields F = C.at(wi.c).F;
