@@ -166,6 +166,10 @@ __device__ __forceinline__ int sweep_done_dirs(const Mesh& M, const mhc_case_par
   return done;
 }
 
+// every item `split` times, for a sweep whose blocks take a share of the
+// variables each
+#define MHC_FOR_SPLIT_ITEMS(L, split) for (int w_ = blockIdx.x; w_ < (L).total * (split); w_ += gridDim.x)
+
 template <int DIM, int NE>
 __global__ void __launch_bounds__(CT) kb_init_cells(const CaseDesc* __restrict__ C, PhaseList L) {
   MHC_FOR_ITEMS(L) {
@@ -328,12 +332,13 @@ __global__ void __launch_bounds__(CT) kb_hourglass(const __grid_constant__ CaseT
 #ifndef MHC_SW_MIN_BLOCKS_PB
 #define MHC_SW_MIN_BLOCKS_PB 4
 #endif
-template <int DIM, int NE, int D, int LIM, int XV = 0, bool SOLO = false>
+// SHARE: `split` blocks per item, each with a share of the variables
+template <int DIM, int NE, int D, int LIM, int XV = 0, bool SOLO = false, bool SHARE = false>
 __global__ void __launch_bounds__(SW_THREADS, LIM == LIM_PB ? MHC_SW_MIN_BLOCKS_PB
                                               : (LIM == LIM_O3 ? MHC_SW_MIN_BLOCKS_O3 : (LIM == LIM_GEN ? 2 : MHC_SW_MIN_BLOCKS_CELLS)))
-kb_sweep_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant__ PhaseList L, int k) {
-  MHC_FOR_ITEMS(L) {
-    const WorkItem wi = item_at<cell_sweep_phase(LIM, D)>(C, L, w_);
+kb_sweep_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant__ PhaseList L, int k, int split) {
+  MHC_FOR_SPLIT_ITEMS(L, SHARE ? split : 1) {
+    const WorkItem wi = item_at<cell_sweep_phase(LIM, D)>(C, L, SHARE ? w_ / split : w_);
     Fields F = C.at(wi.c).F;
     if (!case_active(F)) continue;
     resolve_positions(F);
@@ -348,10 +353,12 @@ kb_sweep_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant_
     A.simple_pente = P.projection_simple_pente;
     // EstMixte / EstPure are zero before the first remap of the run
     A.first_remap = k == 0 && F.s->iteration == 1;
+    A.part = SHARE ? w_ % split : 0;
+    A.parts = split;
     const Mesh M = C.at(wi.c).M;
     if constexpr (LIM == LIM_O3) body_sweep_cells_o3<DIM, NE, D>(M, F, A, wi.x, wi.y);
     else if constexpr (LIM == LIM_PB) body_sweep_cells_pb<DIM, NE, D>(M, F, P, A, wi.x, wi.y);
-    else body_sweep_cells_lanes<DIM, NE, D, LIM, XV>(M, F, A, wi.x, wi.y);
+    else body_sweep_cells_lanes<DIM, NE, D, LIM, SHARE, XV>(M, F, A, wi.x, wi.y);
   }
 }
 
@@ -361,12 +368,12 @@ kb_sweep_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant_
 #ifndef MHC_SWT_MIN_BLOCKS
 #define MHC_SWT_MIN_BLOCKS 4
 #endif
-template <int DIM, int NE, int D, int LIM, bool SOLO = false>
+template <int DIM, int NE, int D, int LIM, bool SOLO = false, bool SHARE = false>
 __global__ void __launch_bounds__(SWT_THREADS, MHC_SWT_MIN_BLOCKS)
-kb_sweep_cells_tile(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant__ PhaseList L, int k) {
+kb_sweep_cells_tile(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant__ PhaseList L, int k, int split) {
   extern __shared__ double swt_tile[];
-  MHC_FOR_ITEMS(L) {
-    const WorkItem wi = item_at<PH_SWCT0 + D>(C, L, w_);
+  MHC_FOR_SPLIT_ITEMS(L, SHARE ? split : 1) {
+    const WorkItem wi = item_at<PH_SWCT0 + D>(C, L, SHARE ? w_ / split : w_);
     Fields F = C.at(wi.c).F;
     if (!case_active(F)) continue;  // uniform over the block (one case per item)
     resolve_positions(F);
@@ -380,8 +387,10 @@ kb_sweep_cells_tile(const __grid_constant__ CaseTable<SOLO> C, const __grid_cons
     A.limiter = P.projection_limiteur_id;
     A.simple_pente = P.projection_simple_pente;
     A.first_remap = k == 0 && F.s->iteration == 1;
+    A.part = SHARE ? w_ % split : 0;
+    A.parts = split;
     const Mesh M = C.at(wi.c).M;
-    body_sweep_cells_tile<DIM, NE, D, LIM>(M, F, A, wi.x, wi.y, swt_tile);
+    body_sweep_cells_tile<DIM, NE, D, LIM, SHARE>(M, F, A, wi.x, wi.y, swt_tile);
   }
 }
 

@@ -27,7 +27,16 @@ struct SweepArgs {
   int limiter;
   int simple_pente;   // projection-simple-pente (generalised limiters)
   int first_remap;    // first remap of the run: every cell counts as pure
+  int part, parts;    // classical limiters: this block sweeps the part-th share of the variables
 };
+
+// the variables [v0, v1) of a share of NV (SHARE: a launch over one case whose
+// blocks split the variables; otherwise all of them)
+template <int NV, bool SHARE>
+__device__ __forceinline__ void share_of(const SweepArgs& A, int& v0, int& v1) {
+  v0 = SHARE ? NV * A.part / A.parts : 0;
+  v1 = SHARE ? NV * (A.part + 1) / A.parts : NV;
+}
 
 // face node q (in the order of the reference face, smallest node id first)
 // of the face normal to D whose lowest node is (i, j, k)
@@ -470,7 +479,7 @@ struct CellLane {
 // ---------------------------------------------------------------------------
 // XV: further projected variables after the pseudo-viscosity (the
 // deviator and plastic strains of an elasto-plastic case), remapped like it
-template <int DIM, int NE, int D, int LIM, int XV = 0>
+template <int DIM, int NE, int D, int LIM, bool SHARE, int XV = 0>
 __device__ __forceinline__ void body_sweep_cells_lanes(const Mesh& M, const Fields& F, const SweepArgs& A,
                                                        int vbx, int vby) {
   constexpr int NV = 3 * NE + 1 + XV;
@@ -517,7 +526,10 @@ __device__ __forceinline__ void body_sweep_cells_lanes(const Mesh& M, const Fiel
     xc = centre_from_planes<DIM, D>(back, front);
     if (out) sweep_normals<DIM, D>(M, p, ta, tb, K.ondB, K.ondF);
   }
-  double u = ok ? __ldg(Uin + c) : 0.;
+  int v0, v1;
+  share_of<NV, SHARE>(A, v0, v1);
+  const double* src = Uin + v0 * N + c;
+  double u = ok ? __ldg(src) : 0.;
   if constexpr (LIM == LIM_GEN) {
     // widths of the own and neighbouring cells
     K.hw = lane_cell_width<DIM, D>(M, F, ok, i, j, k, p, nd);
@@ -535,13 +547,12 @@ __device__ __forceinline__ void body_sweep_cells_lanes(const Mesh& M, const Fiel
   const double xc_l = __shfl_up_sync(FULL, xc, 1);
   K.face_b = ok && ok_l;                       // face between p-1 and p
   K.set_faces(dt, order2, fc, xc, xc_l, un, L, den);
-  const double* src = Uin + c;
-  double* dst = A.Uout + c;
+  double* dst = A.Uout + v0 * N + c;
 #pragma unroll 1
-  for (int v = 0; v < NV; ++v) {
+  for (int v = v0; v < v1; ++v) {
     // the next variable's value is on its way during this one's arithmetic
     src += N;
-    const double u_next = (ok && v + 1 < NV) ? __ldg(src) : 0.;
+    const double u_next = (ok && v + 1 < v1) ? __ldg(src) : 0.;
     double fB, fF;
     K.fluxes(u, fB, fF);
     if (out) {
@@ -1103,7 +1114,7 @@ constexpr int SWT_FIELD = SW_LANES * SWT_PITCH;  // doubles per staged quantity
 __host__ __device__ constexpr int swt_slots(int ne) { return 3 * ne + 1 + 5; }
 __host__ __device__ constexpr int swt_smem_bytes(int ne) { return swt_slots(ne) * SWT_FIELD * 8; }
 
-template <int DIM, int NE, int D, int LIM>
+template <int DIM, int NE, int D, int LIM, bool SHARE>
 __device__ __forceinline__ void body_sweep_cells_tile(const Mesh& M, const Fields& F, const SweepArgs& A, int vbx,
                                                       int vby, double* __restrict__ sm) {
   static_assert(D >= 1, "x sweeps use the lane layout");
@@ -1115,7 +1126,9 @@ __device__ __forceinline__ void body_sweep_cells_tile(const Mesh& M, const Field
   const int x0 = vbx * SWT_COLS;
   const int g0 = vby * XOUT - 2;  // first position of the window (2 halo cells)
   const double* __restrict__ Uin = A.Uin;
-  // -- 1. load (row layout)
+  int v0, v1;
+  share_of<NV, SHARE>(A, v0, v1);
+  // -- 1. load (row layout); the volumes make the divisor of every share
   {
     const int col = threadIdx.x % SWT_COLS, pos = threadIdx.x / SWT_COLS;
     const int i = x0 + col, g = g0 + pos;
@@ -1130,6 +1143,7 @@ __device__ __forceinline__ void body_sweep_cells_tile(const Mesh& M, const Field
       double den = 0.;
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
+        if (v >= NE && (v < v0 || v >= v1)) continue;
         const double u = __ldg(Uin + v * N + c);
         s[v * SWT_FIELD] = u;
         if (v < NE) den += u;
@@ -1175,7 +1189,7 @@ __device__ __forceinline__ void body_sweep_cells_tile(const Mesh& M, const Field
     K.face_b = ok && ok_l;                       // face between p-1 and p
     K.set_faces(dt, order2, fc, xc, xc_l, un, L, den);
 #pragma unroll 1
-    for (int v = 0; v < NV; ++v) {
+    for (int v = v0; v < v1; ++v) {
       const double u = ok ? s[v * SWT_FIELD] : 0.;
       double fB, fF;
       const bool some = K.fluxes(u, fB, fF);
@@ -1199,9 +1213,11 @@ __device__ __forceinline__ void body_sweep_cells_tile(const Mesh& M, const Field
       const long long c = cell_id(M, i, D == 1 ? p : tb, D == 1 ? tb : p);
       const double* s = sm + pos * SWT_PITCH + col;
 #pragma unroll
-      for (int v = 0; v < NV; ++v) A.Uout[v * N + c] = s[v * SWT_FIELD];
+      for (int v = 0; v < NV; ++v)
+        if (v >= v0 && v < v1) A.Uout[v * N + c] = s[v * SWT_FIELD];
 #pragma unroll
-      for (int e = 0; e < NE; ++e) F.mflux[e * N + c] = s[(S_XC + e) * SWT_FIELD];
+      for (int e = 0; e < NE; ++e)
+        if (NE + e >= v0 && NE + e < v1) F.mflux[e * N + c] = s[(S_XC + e) * SWT_FIELD];
     }
   }
   __syncthreads();  // the tile is reused by the block's next work item

@@ -16,25 +16,37 @@ namespace {
 template <int DIM, int LIM>
 void cell_sweep_elasto(Engine* e, Group& g, int D, int k) {
   StageTimer tm(e, MHC_STAGE_SWEEP_CELLS);
-  if (D == 0) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, 1, 0, LIM, MHC_ELASTO_XV, SOLO>), SW_THREADS, 0, g.sw_cells[0], k);
-  else if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, 1, 1, LIM, MHC_ELASTO_XV, SOLO>), SW_THREADS, 0, g.sw_cells[1], k);
-  else if constexpr (DIM == 3) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, 1, 2, LIM, MHC_ELASTO_XV, SOLO>), SW_THREADS, 0, g.sw_cells[2], k);
+  if (D == 0) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, 1, 0, LIM, MHC_ELASTO_XV, SOLO>), SW_THREADS, 0, g.sw_cells[0], k, 1);
+  else if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, 1, 1, LIM, MHC_ELASTO_XV, SOLO>), SW_THREADS, 0, g.sw_cells[1], k, 1);
+  else if constexpr (DIM == 3) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, 1, 2, LIM, MHC_ELASTO_XV, SOLO>), SW_THREADS, 0, g.sw_cells[2], k, 1);
 }
 
+// x sweeps, and the y / z sweeps of the limiters and layouts without a tile
 template <int DIM, int NE, int LIM>
 void cell_sweep(Engine* e, Group& g, int D, int k) {
   StageTimer tm(e, MHC_STAGE_SWEEP_CELLS);
-  if (D == 0) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 0, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[0], k);
-  else if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 1, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[1], k);
-  else if constexpr (DIM == 3) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 2, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[2], k);
+  if (D == 0) {
+    if constexpr (LIM <= LIM_ORDER1)
+      plaunch_cells(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 0, LIM, 0, SOLO>),
+                    MHC_KERNEL(kb_sweep_cells<DIM, NE, 0, LIM, 0, SOLO, SOLO>), SW_THREADS, 0, g.sw_cells[0], 3 * NE + 1, k);
+    else
+      plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 0, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[0], k, 1);
+  } else if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 1, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[1], k, 1);
+  else if constexpr (DIM == 3) plaunch_case(e, MHC_KERNEL(kb_sweep_cells<DIM, NE, 2, LIM, 0, SOLO>), SW_THREADS, 0, g.sw_cells[2], k, 1);
 }
 
 // y / z cell sweeps through the shared-memory tile
+template <int DIM, int NE, int D, int LIM>
+void cell_sweep_tile_dir(Engine* e, Group& g, int k) {
+  plaunch_cells(e, MHC_KERNEL(kb_sweep_cells_tile<DIM, NE, D, LIM, SOLO>),
+                MHC_KERNEL(kb_sweep_cells_tile<DIM, NE, D, LIM, SOLO, SOLO>), SWT_THREADS, swt_smem_bytes(NE),
+                g.sw_cells[D], 3 * NE + 1, k);
+}
 template <int DIM, int NE, int LIM>
 void cell_sweep_tile(Engine* e, Group& g, int D, int k) {
   StageTimer tm(e, MHC_STAGE_SWEEP_CELLS);
-  if (D == 1) plaunch_case(e, MHC_KERNEL(kb_sweep_cells_tile<DIM, NE, 1, LIM, SOLO>), SWT_THREADS, swt_smem_bytes(NE), g.sw_cells[1], k);
-  else if constexpr (DIM == 3) plaunch_case(e, MHC_KERNEL(kb_sweep_cells_tile<DIM, NE, 2, LIM, SOLO>), SWT_THREADS, swt_smem_bytes(NE), g.sw_cells[2], k);
+  if (D == 1) cell_sweep_tile_dir<DIM, NE, 1, LIM>(e, g, k);
+  else if constexpr (DIM == 3) cell_sweep_tile_dir<DIM, NE, 2, LIM>(e, g, k);
 }
 
 // y / z node sweeps through the shared-memory tile
