@@ -832,7 +832,7 @@ int case_alloc(const mhc_case_params* params, cudaStream_t stream, mhc_case** ou
   M.h[0] = params->lx / params->nx;
   M.h[1] = params->ly / params->ny;
   M.h[2] = h->DIM == 3 ? params->lz / params->nz : 0.;
-  M.unit_normals = unit_normals_mask(M);
+  if (params->with_projection) M.unit_normals = unit_normals_mask(M);  // read by the sweeps only
   if (stream) {
     h->stream = stream;
   } else {

@@ -15,6 +15,8 @@
 // are rebuilt from the node positions.  The initial face normals of the
 // cartesian grid are unit axis vectors, so dot(., n) is the D component.
 #pragma once
+#include <vector>
+
 #include "mhc_kernels.cuh"
 
 namespace mhc {
@@ -140,34 +142,43 @@ __host__ __device__ __forceinline__ void outer_normals(const Mesh& M, int p, int
 // from a tiny mesh that the rounding of its coordinates shows.  The sweeps
 // then skip the normals: about 110 of their 390 FP64 operations per cell in
 // 3D with one material (Mesh::unit_normals, evaluated once per case).
+// cc: the initial cell centres along every axis (cc0_comp).
 template <int DIM, int D>
-inline bool outer_normals_unit(const Mesh& M) {
+inline bool outer_normals_unit(const Mesh& M, const std::vector<double> (&cc)[3]) {
   constexpr int A0 = D == 0 ? 1 : 0, A1 = D == 2 ? 1 : 2;
   const int n[3] = {M.ncx, M.ncy, M.ncz};
   double a = 0., b = 0.;
   for (int i = 0; i < n[A0]; ++i) {
-    const double t = fc0_comp<DIM, D, A0>(M, i) - cc0_comp<DIM, A0>(M, i);
+    const double t = fc0_comp<DIM, D, A0>(M, i) - cc[A0][i];
     if (!(t * t <= a)) a = t * t;
   }
   for (int i = 0; i < n[A1]; ++i) {
-    const double t = fc0_comp<DIM, D, A1>(M, i) - cc0_comp<DIM, A1>(M, i);
+    const double t = fc0_comp<DIM, D, A1>(M, i) - cc[A1][i];
     if (!(t * t <= b)) b = t * t;
   }
   for (int p = 0; p < n[D]; ++p) {
-    const double cc0 = cc0_comp<DIM, D>(M, p);
     for (int front = 0; front < 2; ++front) {
-      const double d = fc0_comp<DIM, D, D>(M, p + front) - cc0, dd = d * d;
+      const double d = fc0_comp<DIM, D, D>(M, p + front) - cc[D][p], dd = d * d;
       const double ss = D == 0 ? dd + a + b : (D == 1 ? a + dd + b : a + b + dd);
       if (ss != dd || d / std::sqrt(dd) != (front ? 1. : -1.)) return false;
     }
   }
   return true;
 }
-inline int unit_normals_mask(const Mesh& M) {
-  if (M.dim == 2) return (outer_normals_unit<2, 0>(M) ? 1 : 0) | (outer_normals_unit<2, 1>(M) ? 2 : 0);
-  return (outer_normals_unit<3, 0>(M) ? 1 : 0) | (outer_normals_unit<3, 1>(M) ? 2 : 0) |
-         (outer_normals_unit<3, 2>(M) ? 4 : 0);
+template <int DIM>
+inline int unit_normals_of(const Mesh& M) {
+  std::vector<double> cc[3];
+  cc[0].resize(M.ncx);
+  cc[1].resize(M.ncy);
+  cc[2].resize(M.ncz);
+  for (int i = 0; i < M.ncx; ++i) cc[0][i] = cc0_comp<DIM, 0>(M, i);
+  for (int j = 0; j < M.ncy; ++j) cc[1][j] = cc0_comp<DIM, 1>(M, j);
+  for (int k = 0; k < M.ncz; ++k) cc[2][k] = cc0_comp<DIM, 2>(M, k);
+  int m = (outer_normals_unit<DIM, 0>(M, cc) ? 1 : 0) | (outer_normals_unit<DIM, 1>(M, cc) ? 2 : 0);
+  if constexpr (DIM == 3) m |= outer_normals_unit<3, 2>(M, cc) ? 4 : 0;
+  return m;
 }
+inline int unit_normals_mask(const Mesh& M) { return M.dim == 2 ? unit_normals_of<2>(M) : unit_normals_of<3>(M); }
 
 // the same in the sweeps
 template <int DIM, int D>
