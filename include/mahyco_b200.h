@@ -114,8 +114,8 @@ int mhc_compute_delta_t(mhc_case* h);
 int mhc_cycle(mhc_case* h, int n);
 
 /* same as mhc_cycle, but the iterations are captured once in a CUDA graph
- * (one 6-iteration period, which brings every sweep order back) and
- * replayed; n = 0 right after HydroStartInit captures the graph without
+ * (one period, which brings every sweep order back: 2 iterations of a 2D
+ * remap, 3 of a 3D one, 6 otherwise) and replayed; n = 0 right after HydroStartInit captures the graph without
  * running an iteration */
 int mhc_cycle_graph(mhc_case* h, int n);
 
@@ -284,7 +284,8 @@ int mhc_batch_init(mhc_batch* b);
 /* retire a case and release its device memory */
 int mhc_batch_remove(mhc_batch* b, int index);
 int mhc_batch_cycle(mhc_batch* b, int n);
-/* same, replaying a CUDA graph of 6 iterations (one sweep-rotation period) */
+/* same, replaying a CUDA graph of one sweep-rotation period (2 iterations when
+ * every case is a 2D remap, 3 when every one is 3D, 6 otherwise) */
 int mhc_batch_cycle_graph(mhc_batch* b, int n);
 int mhc_batch_cycle_timed(mhc_batch* b, int n, double* stage_ms, long long* stage_launches);
 int mhc_batch_synchronize(mhc_batch* b);

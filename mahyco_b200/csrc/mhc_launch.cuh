@@ -312,8 +312,9 @@ __global__ void __launch_bounds__(CT) kb_hourglass(const __grid_constant__ CaseT
 
 // k-th performed sweep of the cycle in direction D: U[k&1] -> U[(k+1)&1]
 // resident blocks per SM asked of the compiler for the sweeps (caps their
-// registers at 65536 / (SW_THREADS * value)); measured best on B200: 6 for
-// the cell sweeps (80 registers), 8 for the node sweeps (64 registers)
+// registers at 65536 / (SW_THREADS * value)): 8 (64 registers) for the
+// classical limiters, whose variable loop is rolled; 6 blocks of the same
+// cell sweep are 9 % slower, 10 (48 registers) 11 %
 #ifndef MHC_SW_MIN_BLOCKS_CELLS
 #define MHC_SW_MIN_BLOCKS_CELLS 8
 #endif
@@ -321,9 +322,8 @@ __global__ void __launch_bounds__(CT) kb_hourglass(const __grid_constant__ CaseT
 #define MHC_SW_MIN_BLOCKS_NODES 8
 #endif
 
-// the generalised-limiter and third-order instances hold more state per
-// lane and are asked for fewer resident blocks
-// the third-order sweep: 5 (96 registers; 101x37x35 cells 44 us at 4, 40 at 5);
+// the instances of the wide stencils hold more state per lane and are asked
+// for fewer resident blocks.  The third-order sweep: 5 (96 registers; 101x37x35 cells 44 us at 4, 40 at 5);
 // the pente-borne one: 4 (128 registers; 350x150 cells, three environments: 35
 // us, 5 blocks 38 there and 6 % faster at 1200x500)
 #ifndef MHC_SW_MIN_BLOCKS_O3

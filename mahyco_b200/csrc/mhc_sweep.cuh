@@ -1,5 +1,9 @@
-// mhc_sweep.cuh -- one direction of the ADI remap (cells, then nodes)
-// without shared memory or barriers.
+// mhc_sweep.cuh -- one direction of the ADI remap (cells, then nodes).
+//
+// Two forms of the same arithmetic: the x sweeps (and every sweep of the wide
+// stencils) one warp per line, without shared memory or barriers; the y and z
+// sweeps of the classical limiters through a shared-memory tile that turns
+// their strided lines into runs of consecutive x.
 //
 // A warp holds 32 consecutive cells along the sweep direction, one per
 // lane; every intermediate of the reference -- phi, face gradient, limited
@@ -1460,15 +1464,14 @@ __device__ __forceinline__ void body_sweep_nodes_lanes(const Mesh& M, const Fiel
 // ---------------------------------------------------------------------------
 // Node sweep along D = 1, 2 through a shared-memory tile, classical limiters
 // and first order (the layout of body_sweep_cells_tile): the load layout
-// stages, per node, its position along D, its projected dual variables, the
-// values phi of the limited reconstruction and the mass flux through its
-// front half-plane; warp w then runs the arithmetic of
+// stages, per node, its position along D, the mass flux through its front
+// half-plane, its mass, and per variable the projected dual U and the value
+// that the limited reconstruction uses; warp w then runs the arithmetic of
 // body_sweep_nodes_lanes on column w, in the same order, and the store
 // layout writes the updated variables of the written nodes (NOUT per
 // window).
 // ---------------------------------------------------------------------------
 // staged: x, front mass flux, mass, then U and value of every variable
-// (1: a direction swept before moved the node, so its mass divides)
 constexpr int SWTN_SLOTS = 11;
 constexpr int SWTN_SMEM_BYTES = SWTN_SLOTS * SWT_FIELD * 8;
 
