@@ -381,7 +381,7 @@ def run_ours(args):
         "config": {"workload": WORKLOADS[args.workload][0], "cells": ncell, "nodes": nnode,
                    "materials": p.nb_env, "remap": bool(p.with_projection),
                    "l2": "working set > 126 MB L2, no flush", "parallelism": f"replicas x{world}",
-                   "timing": "K iterations replayed from the case's CUDA graph of one 6-iteration period"},
+                   "timing": "K iterations replayed from the case's CUDA graph of one sweep-rotation period"},
         "status": m["status"],
         "gpu_launches": m["gpu_launches"],
         "roofline": m["roofline"],
@@ -391,7 +391,7 @@ def run_ours(args):
         "clocks": m["clocks"],
         "e2e": {"value": e2e_value, "unit": "cell-cycles/s",
                 "h2d_bytes_per_step": ctypes.sizeof(p) / args.steps, "d2h_bytes_per_step": d2h / args.steps,
-                "timer": "host wall clock; includes case allocation, device init, the graph capture, the status read-back after every 6-iteration period (overlapping the next period) and the final field download into page-locked result buffers allocated before the timed region"},
+                "timer": "host wall clock; includes case allocation, device init, the graph capture, the status read-back after every 6 iterations (overlapping the next 6) and the final field download into page-locked result buffers allocated before the timed region"},
     }
     if world == 1 and not args.no_extras:
         # the other stated configurations, each at its stated size:
