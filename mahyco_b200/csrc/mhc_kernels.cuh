@@ -119,6 +119,18 @@ __device__ __forceinline__ bool case_active(const Fields& F) {
   return s->status == 0 && s->iteration <= s->iteration_limit;
 }
 
+// the same as one decision of the block, for the kernels whose passes hold
+// block barriers.  A flag can rise while a kernel runs (a NaN of the cells'
+// finalize pass beside the last node sweeps; one that another block of the
+// time step of several cases meets), so the threads of a block may read either
+// state; those that left would meet the barriers of another item, another
+// case's among them, while the rest still shares the tile of this one.  Every
+// thread calls it.
+__device__ __forceinline__ bool block_active(const Fields& F) { return __syncthreads_and(case_active(F)); }
+
+// one decision of the warp, for the passes that exchange values by shuffles
+__device__ __forceinline__ bool warp_active(const Fields& F) { return __all_sync(0xffffffffu, case_active(F)); }
+
 // ---------------------------------------------------------------------------
 // equations of state
 // ---------------------------------------------------------------------------

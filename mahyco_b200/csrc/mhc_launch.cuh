@@ -340,7 +340,7 @@ kb_sweep_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant_
   MHC_FOR_SPLIT_ITEMS(L, SHARE ? split : 1) {
     const WorkItem wi = item_at<cell_sweep_phase(LIM, D)>(C, L, SHARE ? w_ / split : w_);
     Fields F = C.at(wi.c).F;
-    if (!case_active(F)) continue;
+    if (!warp_active(F)) continue;
     resolve_positions(F);
     if (k & 1) F.mflux = F.mflux1;
     const mhc_case_params& P = *C.at(wi.c).P;
@@ -375,7 +375,7 @@ kb_sweep_cells_tile(const __grid_constant__ CaseTable<SOLO> C, const __grid_cons
   MHC_FOR_SPLIT_ITEMS(L, SHARE ? split : 1) {
     const WorkItem wi = item_at<PH_SWCT0 + D>(C, L, SHARE ? w_ / split : w_);
     Fields F = C.at(wi.c).F;
-    if (!case_active(F)) continue;  // uniform over the block (one case per item)
+    if (!case_active(F)) continue;  // nothing raises a flag while the cell sweeps run
     resolve_positions(F);
     if (k & 1) F.mflux = F.mflux1;
     const mhc_case_params& P = *C.at(wi.c).P;
@@ -405,7 +405,7 @@ kb_sweep_nodes_tile(const __grid_constant__ CaseTable<SOLO> C, const __grid_cons
   MHC_FOR_ITEMS(L) {
     const WorkItem wi = item_at<PH_SWNT0 + D>(C, L, w_);
     Fields F = C.at(wi.c).F;
-    if (!case_active(F)) continue;  // uniform over the block (one case per item)
+    if (!block_active(F)) continue;
     resolve_positions(F);
     if (k & 1) F.mflux = F.mflux1;
     const Mesh M = C.at(wi.c).M;
@@ -428,7 +428,7 @@ kb_sweep_nodes(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant_
   MHC_FOR_ITEMS(L) {
     const WorkItem wi = item_at<node_sweep_phase(LIM, D)>(C, L, w_);
     Fields F = C.at(wi.c).F;
-    if (!case_active(F)) continue;
+    if (!warp_active(F)) continue;
     resolve_positions(F);
     if (k & 1) F.mflux = F.mflux1;
     const Mesh M = C.at(wi.c).M;
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(CT) kb_delta_t(const __grid_constant__ CaseTab
   constexpr double TOP = 1.7976931348623157e308;
   if constexpr (SOLO) {
     const Fields& F = C.d.F;
-    if (!case_active(F)) return;
+    if (!block_active(F)) return;
     const Mesh& M = C.d.M;
     const mhc_case_params& P = *C.d.P;
     StepEnd E;
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(CT) kb_delta_t(const __grid_constant__ CaseTab
     MHC_FOR_ITEMS(L) {
       const WorkItem wi = item_at<PH_CELLS>(C, L, w_);
       const Fields F = C.at(wi.c).F;
-      if (!case_active(F)) continue;
+      if (!block_active(F)) continue;
       const Mesh M = C.at(wi.c).M;
       const long long c = wi.x * (long long)CT + threadIdx.x;
       double dx = TOP;
