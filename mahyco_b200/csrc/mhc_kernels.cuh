@@ -23,6 +23,9 @@
 namespace mhc {
 
 enum : int { ST_NEG_VOLUME = 1, ST_DT_UNDERFLOW = 2, ST_NAN = 4, ST_STOP = 8 };
+// Scalars::dt_blocks: what a pass that ends the iteration met, above the count
+// of its blocks (at most 2^31 cells / CT)
+enum : unsigned { DT_NAN = 1u << 30, DT_NEG_VOLUME = 1u << 29, DT_COUNT = DT_NEG_VOLUME - 1 };
 
 // time-loop scalars living on the device (so that whole cycles can be
 // replayed from a CUDA graph without host round trips)
@@ -37,7 +40,7 @@ struct Scalars {
   unsigned long long dt_min_bits;  // running min of l/(c+vmax) as ordered bits
   long long iteration_limit;  // last iteration this case may run
   int status;        // ST_* flags
-  unsigned dt_blocks;  // blocks of the CFL reduction that are done (bit 30: one met a NaN)
+  unsigned dt_blocks;  // blocks of the CFL reduction that are done, and the DT_* notes of the pass
   unsigned int eref_first[4];  // Mie-Gruneisen, energie-ref 0: the first cell (reference order) of
                                // each environment with a nonzero initial energy
 };
@@ -1385,8 +1388,10 @@ __device__ __forceinline__ void advance_temperature(const mhc_env_params& o, dou
 }
 
 // A Lagrangian run's characteristic length and sound speed come back in
-// l_out and c_out for the time step (not set beyond the last cell).
-template <int DIM, int NE, bool EULER, bool EL = false, bool CSTS = false>
+// l_out and c_out for the time step (not set beyond the last cell).  DT: the
+// pass goes on to delta_t_block, which turns its negative volumes into the
+// status.
+template <int DIM, int NE, bool EULER, bool EL = false, bool CSTS = false, bool DT = false>
 __device__ __forceinline__ void body_lagrange_cells(const Mesh& M, const mhc_case_params& P, const Fields& F, int bx,
                                                     double& l_out, double& c_out) {
   constexpr bool GEO = EL || CSTS;
@@ -1411,7 +1416,10 @@ __device__ __forceinline__ void body_lagrange_cells(const Mesh& M, const mhc_cas
     V = cell_volume<DIM>(coord, cqs);
     for (int q = 0; q < NBN; ++q) cqn[q] = load_cqs_rw<DIM>(F, N, c, q);
     store_cqs<DIM>(F, N, c, cqs);
-    if (V < 0.) atomicOr(&F.s->status, ST_NEG_VOLUME);
+    if (V < 0.) {
+      if constexpr (DT) atomicOr(&F.s->dt_blocks, DT_NEG_VOLUME);
+      else atomicOr(&F.s->status, ST_NEG_VOLUME);
+    }
     l = char_length(P, DIM, V, coord);
   } else {
     V = F.V[c];
@@ -2303,9 +2311,10 @@ __device__ __forceinline__ void end_iteration(const StepEnd& E, Scalars* s, bool
 // one block's share of the reduction (every thread of the block calls it; dx
 // of a thread without a cell is the largest double): its minimum goes into
 // dt_min_bits, and the last of the case's `blocks` blocks ends the iteration,
-// with the other scalars it needs loaded ahead (E).  A NaN is only flagged
-// once all blocks are done, and not over an error that the pass itself
-// raised; with a flag set the iteration does not end.
+// with the other scalars it needs loaded ahead (E).  A NaN and a negative
+// volume of the same pass are noted beside the count and only become the
+// case's status once all blocks are done, so that none finds the case retired
+// before the others; with a flag set the iteration does not end.
 __device__ __forceinline__ void delta_t_block(const mhc_case_params& P, const Fields& F, const StepEnd& E, double dx,
                                               bool bad, unsigned blocks) {
   for (int o = 16; o > 0; o >>= 1) dx = fmin(dx, __shfl_xor_sync(0xffffffffu, dx, o));
@@ -2316,21 +2325,18 @@ __device__ __forceinline__ void delta_t_block(const mhc_case_params& P, const Fi
 #pragma unroll
   for (int w = 1; w < CT / 32; ++w) dx = fmin(dx, red[w]);
   Scalars* s = F.s;
-  constexpr unsigned BAD = 1u << 30;
   // (a block whose minimum is not below the one already there adds nothing)
   const unsigned long long own = (unsigned long long)__double_as_longlong(dx);
   if (own < E.min_seen) atomicMin(&s->dt_min_bits, own);
-  if (any_bad) atomicOr(&s->dt_blocks, BAD);
+  if (any_bad) atomicOr(&s->dt_blocks, DT_NAN);
   __threadfence();
   const unsigned done = atomicAdd(&s->dt_blocks, 1u);
-  if ((done & (BAD - 1)) != blocks - 1) return;
+  if ((done & DT_COUNT) != blocks - 1) return;
   __threadfence();
-  const int status = *(volatile int*)&s->status;
   const unsigned long long bits = *(volatile unsigned long long*)&s->dt_min_bits;
-  if (status == 0) {
-    if (done & BAD) s->status = ST_NAN;
-    else end_iteration(E, s, P.deltat_constant, P.deltat_init, bits);
-  }
+  if (done & DT_NEG_VOLUME) s->status = ST_NEG_VOLUME;
+  else if (done & DT_NAN) s->status = ST_NAN;
+  else end_iteration(E, s, P.deltat_constant, P.deltat_init, bits);
   s->dt_blocks = 0;
 }
 

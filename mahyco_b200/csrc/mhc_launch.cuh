@@ -268,7 +268,10 @@ __global__ void __launch_bounds__(CT, MHC_GEOM_MIN_BLOCKS) kb_lagrange_geom(cons
 // from the length and sound speed still in registers and the velocities the
 // node pass left; the last block ends the iteration.  A pass of its own and
 // one more kernel for the scalars took 6.4 of the 21.0 us of an iteration on
-// 200 x 10 cells.  The entry points called one by one keep kb_delta_t.
+// 200 x 10 cells.  The entry points called one by one keep kb_delta_t.  No
+// flag rises while it runs (a negative volume goes into dt_blocks), so the
+// threads of a block agree on case_active and meet at the time step's
+// barriers; one more barrier to decide it took 2 % of an elasto iteration.
 template <int DIM, int NE, bool EULER, bool EL, bool CSTS = false, bool DT = false, bool SOLO = false>
 __global__ void __launch_bounds__(CT, EL || CSTS ? MHC_LAG_MIN_BLOCKS_GEO : MHC_LAG_MIN_BLOCKS) kb_lagrange_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant__ PhaseList L) {
   MHC_FOR_ITEMS(L) {
@@ -287,7 +290,7 @@ __global__ void __launch_bounds__(CT, EL || CSTS ? MHC_LAG_MIN_BLOCKS_GEO : MHC_
       if (c < M.ncell) vmax = cell_vmax<DIM, false>(M, P, F, c);
     }
     double l = 0., cs = 0.;
-    body_lagrange_cells<DIM, NE, EULER, EL, CSTS>(M, P, F, wi.x, l, cs);
+    body_lagrange_cells<DIM, NE, EULER, EL, CSTS, DT>(M, P, F, wi.x, l, cs);
     if constexpr (DT) {
       double dx = 1.7976931348623157e308;
       if (c < M.ncell) dx = l / (cs + vmax);

@@ -56,8 +56,8 @@ def _kernels():
 
 # threads that leave an item by their own reading of the case's state
 ALONE = r"\bcase_active\(\w+\)\)\s*(continue|return)"
-# the kernels that they may in: one case alone (the time step of the cell pass),
-# or no flag that rises while they run (beside the cell sweeps only node sweeps do)
+# the kernels that they may in, since nothing raises a flag while they run: the
+# cell pass (below) and the cell sweeps, beside which only node sweeps run
 QUIET = {"kb_lagrange_cells", "kb_sweep_cells_tile"}
 
 
@@ -77,6 +77,14 @@ def test_shuffles_follow_a_decision_of_the_warp_or_block():
     for k in shuffled - QUIET:
         own = kernels[k][1]
         assert re.search(r"\b(warp|block)_active\(", own) and not re.search(ALONE, own), k
+
+
+def test_cell_pass_raises_no_flag_before_its_time_step_ends():
+    """With the time step in it (DT) the pass notes its negative volumes beside the block count."""
+    body = _functions(_text(), "body_lagrange_")["body_lagrange_cells"]
+    assert body.count("status") == 1
+    assert re.search(r"if constexpr \(DT\)[^;]*dt_blocks[^;]*;\s*else atomicOr\(&F\.s->status", body)
+    assert "body_lagrange_cells<DIM, NE, EULER, EL, CSTS, DT>" in _kernels()["kb_lagrange_cells"][1]
 
 
 def test_sweeps_raise_no_flag():
