@@ -7,7 +7,7 @@ no sound speed.  The healthy cases equal their solo runs bit for bit."""
 import numpy as np
 import pytest
 
-from mahyco_b200.cases import SUPERBEE, VANLEER, seeded_two_state, sod
+from mahyco_b200.cases import SUPERBEE, VANLEER, bar_impact, seeded_two_state, sod
 
 FIELDS = ("Density", "Pressure", "InternalEnergy", "SoundSpeed", "CellMass", "Velocity", "NodeMass")
 
@@ -69,3 +69,24 @@ def test_failing_cases_leave_neighbours_intact(mix, scale):
                 assert s["status"] == 0 and s["iteration"] == n, s
                 for f in FIELDS:
                     assert np.array_equal(b.field(i, f), ref[f]), (i, f)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,deltat", [((16, 8), 1e-4), ((9, 31), 1e-5), ((80, 40), 1e-5)])
+def test_negative_volume_of_the_cell_pass_is_the_status(n, deltat):
+    """An elasto-plastic case whose first time step turns cells over: the same
+    status, iteration and time through the entry points (the geometry raises
+    the flag) and whole iterations (the last block of the pass does), at one
+    block and several, and again after a restart."""
+    from mahyco_b200 import Hydro, ST_NEG_VOLUME
+    for how in ("entry points", "cycle", "graph"):
+        with Hydro(bar_impact(n=n, L=(0.01, 0.03), deltat_init=deltat)) as h:
+            for _ in range(2):
+                h.hydroStartInit()
+                if how == "entry points":
+                    for _ in range(4):
+                        h.iterate()
+                else:
+                    h.cycle(4, graph=how == "graph")
+                s = h.scalars()
+                assert s["status"] == ST_NEG_VOLUME and s["iteration"] == 0, (how, s)
