@@ -13,6 +13,7 @@
 
 #include "../../include/mahyco_b200.h"
 #include "mhc_launch.cuh"
+#include "mhc_resident.h"
 
 namespace mhc {
 
@@ -269,17 +270,16 @@ inline int skip_mask(const mhc_case* h) {
   return m;
 }
 
-// persistent grid for a kernel: resident blocks on the device (cached)
+// persistent grid for a kernel: resident blocks on the device
 template <class K>
 inline int resident_blocks(Engine* e, K kernel, int threads, size_t smem) {
-  static std::map<const void*, int> cache;
-  auto it = cache.find((const void*)kernel);
-  if (it != cache.end()) return it->second * e->nsm;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  cache[(const void*)kernel] = per_sm;
-  return per_sm * e->nsm;
+  static ResidentBlocks cache;
+  return e->nsm * cache.get((const void*)kernel, threads, smem, [&] {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
+      per_sm = 1;
+    return per_sm;
+  });
 }
 
 template <class K, class... Args>
