@@ -5,14 +5,15 @@ arithmetic, so the tuning cycles are ordinary cycles of the run and the
 results are bit-identical whatever the tuner picks:
 
 * the layout of the y / z remap sweeps of classical-limiter cases, for
-  cells and for nodes: one warp per line (lanes along the sweep) or a
+  cells and for nodes: 1, one warp per line (lanes along the sweep), or 2, a
   shared-memory tile (coalesced row loads, the warp-per-line arithmetic on
-  staged values); layout 3, once one thread per line chunk, is the tile
-  again;
+  staged values).  An installed decision may also say 0 or 3, the tile again;
 * the grid of every phase's work-list launch: 0 launches one block per work
   item and lets the hardware balance them, k > 0 launches k times the blocks
   the device holds at once, persistent blocks striding over the list (the
-  one cross-block reduction, the CFL minimum, is order-independent).
+  one cross-block reduction, the CFL minimum, is order-independent).  The
+  time step of a case run alone strides over its cells in either form: its
+  grid is the device's blocks once for 0, k times for k.
 
 The tuner times each candidate over a few cycles with CUDA events around
 every phase (cycle_timed) and installs the fastest per phase.  Decisions
@@ -32,7 +33,7 @@ import math
 import os
 
 CANDIDATES = (0, 1, 2, 4, 8)
-LAYOUTS = {1: "warp-per-line", 2: "tile", 3: "tile (3)"}
+LAYOUTS = {1: "warp-per-line", 2: "tile"}
 
 
 def cache_path() -> str:
@@ -92,7 +93,7 @@ def tune(target, params_list=None, cycles_per_trial: int = 2, candidates=CANDIDA
     install the fastest choices.  With `params_list` (the cases' parameters)
     and a cached decision for their bucket, that decision is installed
     without measuring.  Otherwise every candidate runs `cycles_per_trial`
-    cycles: 3 sweep layouts, then len(candidates) grid scales.  Returns
+    cycles: both sweep layouts, then len(candidates) grid scales.  Returns
     {"bucket", "best": {phase: scale}, "cell_layout", "node_layout",
     "ms_per_launch", "cached"}."""
     key = bucket(params_list) if params_list is not None else None
