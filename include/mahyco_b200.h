@@ -290,7 +290,8 @@ int mhc_batch_cycle_graph(mhc_batch* b, int n);
 int mhc_batch_cycle_timed(mhc_batch* b, int n, double* stage_ms, long long* stage_launches);
 int mhc_batch_synchronize(mhc_batch* b);
 /* launch grid of the phases: 0 (default) = one block per work item,
- * k > 0 = k x the blocks the device can hold at once, striding the list */
+ * k > 0 = k x the blocks the device can hold at once, striding the list (the
+ * time step of a case run alone: the device once for 0, k times for k) */
 int mhc_batch_set_grid_scale(mhc_batch* b, int scale);
 /* per-phase override of the grid scale (stage = enum mhc_stage, scale -1 =
  * back to the batch-wide value); the autotuner sets these */

@@ -47,13 +47,12 @@ struct WorkItem {
 enum PhaseKind {
   PH_CELLS = 0,      // one block per CT cells
   PH_NODES = 1,      // one block per CT nodes
-  PH_UNUSED = 2,
-  PH_SWC0 = 3,       // cell sweep along D = PH - PH_SWC0
-  PH_SWN0 = 6,       // node sweep along D = PH - PH_SWN0
-  PH_SWCW0 = 9,      // cell sweep with the wide (third-order) stencil
-  PH_SWNW0 = 12,     // node sweep with the wide (generalised limiter) stencil
-  PH_SWCT0 = 15,     // cell sweep along D = 1, 2 through a shared-memory tile
-  PH_SWNT0 = 18      // node sweep along D = 1, 2 through a shared-memory tile
+  PH_SWC0 = 2,       // cell sweep along D = PH - PH_SWC0
+  PH_SWN0 = 5,       // node sweep along D = PH - PH_SWN0
+  PH_SWCW0 = 8,      // cell sweep with the wide (third-order) stencil
+  PH_SWNW0 = 11,     // node sweep with the wide (generalised limiter) stencil
+  PH_SWCT0 = 14,     // cell sweep along D = 1, 2 through a shared-memory tile
+  PH_SWNT0 = 17      // node sweep along D = 1, 2 through a shared-memory tile
 };
 
 // phase of the cell sweep along D for a cell-sweep instance
@@ -326,9 +325,12 @@ __global__ void __launch_bounds__(CT) kb_hourglass(const __grid_constant__ CaseT
 #endif
 
 // the instances of the wide stencils hold more state per lane and are asked
-// for fewer resident blocks.  The third-order sweep: 5 (96 registers; 101x37x35 cells 44 us at 4, 40 at 5);
-// the pente-borne one: 4 (128 registers; 350x150 cells, three environments: 35
-// us, 5 blocks 38 there and 6 % faster at 1200x500)
+// for fewer resident blocks.  The third-order sweep: 5 (96 registers; 101x37x35 cells 44 us at 4, 40 at 5).
+// The pente-borne one: 4 (128 registers) against 5 (96, which spill): up to
+// some 2e5 cells a sweep is one wave or two, as long as one warp's chain, and
+// the spills lengthen it (three environments, us a sweep, 4 and 5 blocks:
+// 55x24 32.1 and 34.2, 220x95 34.2 and 37.0, 500x215 43.9 and 48.5, 690x290
+// 66.9 and 67.7); with many waves the fifth block pays (1200x500 187 and 182).
 #ifndef MHC_SW_MIN_BLOCKS_O3
 #define MHC_SW_MIN_BLOCKS_O3 5
 #endif
@@ -351,7 +353,6 @@ kb_sweep_cells(const __grid_constant__ CaseTable<SOLO> C, const __grid_constant_
     A.Uin = (k & 1) ? F.U[1] : F.U[0];
     A.Uout = (k & 1) ? F.U[0] : F.U[1];
     A.first = k == 0;
-    A.order = P.ordre_projection;
     A.limiter = P.projection_limiteur_id;
     A.simple_pente = P.projection_simple_pente;
     // EstMixte / EstPure are zero before the first remap of the run
@@ -386,7 +387,6 @@ kb_sweep_cells_tile(const __grid_constant__ CaseTable<SOLO> C, const __grid_cons
     A.Uin = (k & 1) ? F.U[1] : F.U[0];
     A.Uout = (k & 1) ? F.U[0] : F.U[1];
     A.first = k == 0;
-    A.order = P.ordre_projection;
     A.limiter = P.projection_limiteur_id;
     A.simple_pente = P.projection_simple_pente;
     A.first_remap = k == 0 && F.s->iteration == 1;

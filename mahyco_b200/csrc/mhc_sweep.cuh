@@ -29,7 +29,6 @@ struct SweepArgs {
   const double* Uin;
   double* Uout;
   int first;
-  int order;
   int limiter;
   int simple_pente;   // projection-simple-pente (generalised limiters)
   int first_remap;    // first remap of the run: every cell counts as pure
