@@ -460,7 +460,7 @@ def run_batch(args):
     import ctypes
     import torch
     import mahyco_b200 as mb
-    from mahyco_b200.autotune import tune, CANDIDATES
+    from mahyco_b200.autotune import tune, trial_cycles
     rank = int(os.environ.get("RANK", "0"))
     world = int(os.environ.get("WORLD_SIZE", "1"))
     local = int(os.environ.get("LOCAL_RANK", "0"))
@@ -477,7 +477,7 @@ def run_batch(args):
     sizes = [lib.mhc_case_device_bytes(ctypes.byref(p)) for p in all_cases]
     mine = partition_by_bytes(sizes, world)[rank]
     cases = [all_cases[i] for i in mine]
-    tune_cycles = 2 * (len(CANDIDATES) + 3)
+    tune_cycles = trial_cycles(2)
     warm = max(args.warmup, tune_cycles + 4)
     limit = warm + args.steps
     cells = sum(p.ncell for p in cases)

@@ -88,6 +88,11 @@ def install(target, decision: dict) -> None:
         target.set_stage_grid_scale(stage, scale)
 
 
+def trial_cycles(cycles_per_trial: int = 2, candidates=CANDIDATES) -> int:
+    """Cycles of the run that a `tune` without a cached decision advances."""
+    return cycles_per_trial * (len(LAYOUTS) + len(candidates))
+
+
 def tune(target, params_list=None, cycles_per_trial: int = 2, candidates=CANDIDATES, use_cache: bool = True) -> dict:
     """Tune a batch (mahyco_b200.Batch) or a case run alone (Hydro) and
     install the fastest choices.  With `params_list` (the cases' parameters)
