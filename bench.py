@@ -562,7 +562,7 @@ def run_batch(args):
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64",
         "data": "synthetic",
         "config": {"workload": WORKLOADS["batch2d"][0], "cases": len(all_cases), "cells": total_cells,
-                   "step": "one cycle of every case", "graph": "CUDA graph of 6 cycles",
+                   "step": "one cycle of every case", "graph": "CUDA graph of one sweep-rotation period",
                    "l2": "working set > 126 MB L2, no flush",
                    "parallelism": f"cases shared by device bytes over {world} GPU(s)" if world > 1 else "1 GPU",
                    "cases_gathered": len(gathered) if gathered is not None else None},
