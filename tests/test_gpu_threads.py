@@ -61,7 +61,7 @@ def test_threads_with_their_own_cases():
         except Exception as e:  # reported below, in the test's own thread
             errors.append((q, repr(e)))
 
-    threads = [threading.Thread(target=work, args=(q,)) for q in range(len(jobs))]
+    threads = [threading.Thread(target=work, args=(q,), daemon=True) for q in range(len(jobs))]
     for t in threads:
         t.start()
     for t in threads:
